@@ -11,26 +11,13 @@
 // the FP64 dot products the drivers need (moments, alpha, beta, norms).
 // Channel semantics: channels.py:58-132 (diagonal delta n + V n n, sigma^x
 // amplitude Omega/2 into |r>, conj(Omega)/2 into |g>).
-#include "el_internal.cuh"
+#include "el_apply.cuh"
 
 #include <algorithm>
 
 namespace {
 
-using el::fail;
-
-template <typename S>
-struct HamArgs {
-  const S *diagV;
-  S delta[EL_MAX_SITES];
-  S up_re[EL_MAX_SITES];  // amplitude into a row whose bit k is 1: Omega/2
-  S up_im[EL_MAX_SITES];  // (into a row whose bit k is 0: conj(Omega)/2)
-  const ExPair *px;       // exchange channels (generic kernel only)
-  int npx;
-  int lossy;              // loss diagonal present (generic kernel only)
-  int real_amp;           // every sigma^x amplitude is real (row kernel: cheaper complex FMAs)
-  S loss[EL_MAX_SITES];   // imaginary diagonal per set bit: -gamma/2 (evolution units)
-};
+using namespace el;
 
 // Amplitude <row|H|row ^ (bit bi | bit bj)> of exchange pair e for a row whose
 // bits at bi, bj are (si, sj): J channel (channels.py:121-125) when the bits
@@ -41,22 +28,6 @@ __device__ __forceinline__ void exchange_amp(const ExPair &e, bool si, bool sj,
   if (si != sj) { re = e.jre; im = si ? e.jim : -e.jim; }
   else { re = e.are; im = si ? e.aim : -e.aim; }
 }
-
-struct KArgs {
-  int64_t nvec;
-  int lognv;
-  const void *x;
-  const void *z;
-  void *y;
-  void *acc;
-  double a, b, c, w_re, w_im;
-  double *dots;
-  int want;
-  int skip_diag;
-  const void *probe;
-  double *partials;
-  unsigned int *counter;
-};
 
 template <typename S, bool C> struct Val;
 template <typename S> struct Val<S, false> {
@@ -72,21 +43,34 @@ template <typename S> struct Val<S, true> {
   __device__ void store(void *p, int64_t i) const { ((S *)p)[2 * i] = re; ((S *)p)[2 * i + 1] = im; }
 };
 
-// Block reduction of 4 doubles per thread into per-(vector, quantity) sums,
-// then a deterministic cross-block sum by the last block to finish.
+// Block reduction of 4 doubles per thread into per-(vector, quantity) sums
+// (thread t holds vector t mod nvec; nvec divides 256), then a deterministic
+// cross-block sum by the last block to finish.  Lanes that hold the same
+// vector meet in a butterfly of shuffles, warps through shared memory; the
+// last block gives every output 256 / nout threads, each adding every
+// (256 / nout)-th block in order.  Both tails are latency chains: with four
+// threads adding 256 values of the block and then one per block in turn, an
+// FP64 product with dots on 65,536 rows took 34.1 us of which the product is
+// 9 us; this form takes 10.2 us.
 __device__ void reduce4(const KArgs &K, double q0, double q1, double q2, double q3) {
   __shared__ double red[256][4];
   __shared__ bool last;
   const int tid = threadIdx.x;
+  const int nv = (int)K.nvec;
+  const int nout = nv * 4;
+  for (int o = 16; o >= nv; o >>= 1) {
+    q0 += __shfl_xor_sync(0xffffffffu, q0, o);
+    q1 += __shfl_xor_sync(0xffffffffu, q1, o);
+    q2 += __shfl_xor_sync(0xffffffffu, q2, o);
+    q3 += __shfl_xor_sync(0xffffffffu, q3, o);
+  }
   red[tid][0] = q0; red[tid][1] = q1; red[tid][2] = q2; red[tid][3] = q3;
   __syncthreads();
-  const int nv = (int)K.nvec;            // nvec divides 256
-  const int per = 256 / nv;
-  const int nout = nv * 4;
+  const int step = nv < 32 ? 32 : nv;    // one value per warp below 32 vectors
   for (int o = tid; o < nout; o += 256) {
     const int v = o >> 2, q = o & 3;
     double s = 0.0;
-    for (int j = 0; j < per; ++j) s += red[v + j * nv][q];
+    for (int j = v; j < 256; j += step) s += red[j][q];
     K.partials[(size_t)blockIdx.x * nout + o] = s;
   }
   __threadfence();
@@ -95,10 +79,25 @@ __device__ void reduce4(const KArgs &K, double q0, double q1, double q2, double 
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int o = tid; o < nout; o += 256) {
+  if (nout <= 128) {
+    // tid = share * nout + output: neighbours read neighbouring outputs
+    const int per = 256 / nout, o = tid & (nout - 1), sh = tid / nout;
     double s = 0.0;
-    for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(&K.partials[(size_t)b * nout + o]);
-    K.dots[o] = s;
+    for (unsigned b = sh; b < gridDim.x; b += per) s += __ldcg(&K.partials[(size_t)b * nout + o]);
+    double *flat = &red[0][0];
+    flat[tid] = s;
+    __syncthreads();
+    for (int w = per >> 1; w > 0; w >>= 1) {
+      if (sh < w) flat[tid] += flat[tid + w * nout];
+      __syncthreads();
+    }
+    if (sh == 0) K.dots[o] = flat[tid];
+  } else {
+    for (int o = tid; o < nout; o += 256) {
+      double s = 0.0;
+      for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(&K.partials[(size_t)b * nout + o]);
+      K.dots[o] = s;
+    }
   }
   if (tid == 0) *K.counter = 0u;
 }
@@ -591,337 +590,6 @@ __global__ void __launch_bounds__(256) k_apply_row(BasisDev B, HamArgs<S> H, KAr
   if constexpr (WANT) reduce4(K, q0, q1, q2, q3);
 }
 
-// ------------------------------------------- chain tile kernel (CHAIN layout)
-// Rows of a nearest-neighbour chain sector that share the code bits >= L form
-// one contiguous block of F(L+2) rows (F(L+1) when bit L is set), ordered by
-// the low L bits exactly like the L-site chain itself.  A CTA takes one such
-// block (a tile) at a time:
-//   - flips of low bits k < L stay inside the tile: the tile of x is staged
-//     in shared memory and the partner is row +- F(k+2) of the same tile;
-//   - a flip of a high bit k >= L moves the whole tile by +- F(k+2) rows (the
-//     low part is unchanged), and whether it is allowed depends only on the
-//     tile's prefix (for k = L and bit L clear: on the tile's first F(L+1)
-//     rows), so it is a contiguous, coalesced read of x with one amplitude
-//     for the tile.
-// Low codes and their detuning sums are tabulated once per CTA in shared
-// memory.  Same fused epilogue as the row kernel.
-
-// Streaming (evict-first) row access for vectors that are touched once per
-// launch (y, z, acc), so that L2 keeps x, whose rows are re-read as flip
-// partners by other tiles.
-template <typename S, int W>
-__device__ __forceinline__ void ld_row_cs(const S *p, S (&v)[W]) {
-  constexpr int BYTES = W * (int)sizeof(S);
-  if constexpr (BYTES % 16 == 0) {
-    union { uint4 u[BYTES / 16]; S s[W]; } t;
-#pragma unroll
-    for (int i = 0; i < BYTES / 16; ++i) t.u[i] = __ldcs(reinterpret_cast<const uint4 *>(p) + i);
-#pragma unroll
-    for (int i = 0; i < W; ++i) v[i] = t.s[i];
-  } else if constexpr (BYTES == 8) {
-    union { uint2 u; S s[W]; } t;
-    t.u = __ldcs(reinterpret_cast<const uint2 *>(p));
-#pragma unroll
-    for (int i = 0; i < W; ++i) v[i] = t.s[i];
-  } else {
-#pragma unroll
-    for (int i = 0; i < W; ++i) v[i] = __ldcs(p + i);
-  }
-}
-
-template <typename S, int W>
-__device__ __forceinline__ void st_row_cs(S *p, const S (&v)[W]) {
-  constexpr int BYTES = W * (int)sizeof(S);
-  if constexpr (BYTES % 16 == 0) {
-    union { uint4 u[BYTES / 16]; S s[W]; } t;
-#pragma unroll
-    for (int i = 0; i < W; ++i) t.s[i] = v[i];
-#pragma unroll
-    for (int i = 0; i < BYTES / 16; ++i) __stcs(reinterpret_cast<uint4 *>(p) + i, t.u[i]);
-  } else if constexpr (BYTES == 8) {
-    union { uint2 u; S s[W]; } t;
-#pragma unroll
-    for (int i = 0; i < W; ++i) t.s[i] = v[i];
-    __stcs(reinterpret_cast<uint2 *>(p), t.u);
-  } else {
-#pragma unroll
-    for (int i = 0; i < W; ++i) __stcs(p + i, v[i]);
-  }
-}
-
-// Shared tile of x: rows of more than 16 bytes are stored chunk-major
-// ([16-byte chunk][row]) so that the 16-byte loads of a warp's 32 rows hit
-// 32 consecutive chunks instead of a 4- or 8-way bank conflict.
-template <typename S, int W>
-__device__ __forceinline__ void tile_ld(const S *xt, int ts, int row, S (&v)[W]) {
-  constexpr int BYTES = W * (int)sizeof(S);
-  if constexpr (BYTES > 16 && BYTES % 16 == 0) {
-    union { uint4 u[BYTES / 16]; S s[W]; } t;
-#pragma unroll
-    for (int i = 0; i < BYTES / 16; ++i) t.u[i] = reinterpret_cast<const uint4 *>(xt)[(size_t)i * ts + row];
-#pragma unroll
-    for (int i = 0; i < W; ++i) v[i] = t.s[i];
-  } else {
-    ld_row<S, W>(xt + (size_t)row * W, v);
-  }
-}
-
-struct TileFlip {
-  int64_t off;   // row offset of the partner
-  int32_t len;   // rows [0, len) of the tile have this flip
-  int32_t k;     // bit
-};
-
-// RA: the amplitudes are real (real Omega) although the vectors are
-// complex: two FMAs per complex entry instead of four.
-template <typename S, bool C, int NV, bool RA = false>
-__device__ __forceinline__ void acc_flip(S (&h)[NV * (C ? 2 : 1)], S are, S aim,
-                                         const S (&xv)[NV * (C ? 2 : 1)]) {
-  if constexpr (C && RA) {
-#pragma unroll
-    for (int v = 0; v < 2 * NV; ++v) h[v] += are * xv[v];
-  } else if constexpr (C) {
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      h[2 * v] += are * xv[2 * v] - aim * xv[2 * v + 1];
-      h[2 * v + 1] += are * xv[2 * v + 1] + aim * xv[2 * v];
-    }
-  } else {
-#pragma unroll
-    for (int v = 0; v < NV; ++v) h[v] += are * xv[v];
-  }
-}
-
-template <typename S, bool C, int NV, bool WANT, bool RA>
-__global__ void __launch_bounds__(256) k_apply_chain_tile(BasisDev B, HamArgs<S> H, KArgs K, int L,
-                                                          int64_t ntiles) {
-  constexpr int W = NV * (C ? 2 : 1);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n = B.n;
-  const int TS = (int)B.fib[L + 2];                       // rows of a full tile
-  // [TS][W] tile of x, then the S-typed table, then the 4-byte table, so
-  // every array starts on a boundary of its element size
-  S *xt = reinterpret_cast<S *>(smem_raw);
-  S *ld = xt + (size_t)TS * W;                            // low detuning sums
-  uint32_t *lc = reinterpret_cast<uint32_t *>(ld + TS);   // low codes
-  __shared__ TileFlip hf[EL_MAX_SITES];
-  __shared__ S hf_re[EL_MAX_SITES], hf_im[EL_MAX_SITES];
-  __shared__ int nhf;
-  __shared__ int s_w[EL_MAX_SITES];            // F(k+2) of the low bits
-  __shared__ S s_are[EL_MAX_SITES], s_aim[EL_MAX_SITES];
-  __shared__ uint32_t s_amp;                    // low bits with a nonzero amplitude
-  __shared__ int64_t t_base;
-  __shared__ int t_size;
-  __shared__ int t_bl;       // bit L of the tile's prefix
-  __shared__ S t_delta;      // detuning sum of the prefix bits
-  for (int k = threadIdx.x; k < L; k += blockDim.x) {
-    s_w[k] = (int)B.fib[k + 2];
-    s_are[k] = H.up_re[k];
-    s_aim[k] = C ? H.up_im[k] : S(0);
-  }
-  if (threadIdx.x == 0) {
-    uint32_t am = 0;
-    for (int k = 0; k < L; ++k)
-      if (H.up_re[k] != S(0) || (C && H.up_im[k] != S(0))) am |= 1u << k;
-    s_amp = am;
-  }
-  // low codes of the L-site chain in ascending order, and their detunings
-  for (int i = threadIdx.x; i < TS; i += blockDim.x) {
-    uint32_t c = 0;
-    int64_t r = i;
-    for (int k = L - 1; k >= 0; --k) {
-      const int64_t w = (int64_t)B.fib[k + 2];
-      if (r >= w) { c |= 1u << k; r -= w; }
-    }
-    lc[i] = c;
-    S d = S(0);
-    for (int k = 0; k < L; ++k)
-      if ((c >> k) & 1u) d += H.delta[k];
-    ld[i] = d;
-  }
-  const S *__restrict__ xp = (const S *)K.x;
-  double q0 = 0, q1 = 0, q2 = 0, q3 = 0;
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    __syncthreads();   // tables ready; previous tile done with xt / hf
-    if (threadIdx.x == 0) {
-      // prefix of tile t: the (n-L)-site chain code of rank t
-      uint64_t p = 0;
-      int64_t r = t;
-      for (int j = n - L - 1; j >= 0; --j) {
-        const int64_t w = (int64_t)B.fib[j + 2];
-        if (r >= w) { p |= 1ULL << j; r -= w; }
-      }
-      int64_t base = 0;
-      S dp = S(0);
-      for (int j = 0; j < n - L; ++j)
-        if ((p >> j) & 1ULL) { base += (int64_t)B.fib[L + j + 2]; dp += H.delta[L + j]; }
-      const int bl = (int)(p & 1ULL);
-      const int size = bl ? (int)B.fib[L + 1] : TS;
-      int cnt = 0;
-      for (int j = 0; j < n - L; ++j) {
-        const int k = L + j;
-        const S are = H.up_re[k];
-        const bool set = (p >> j) & 1ULL;
-        const S aim = C ? (set ? H.up_im[k] : -H.up_im[k]) : S(0);
-        if (are == S(0) && aim == S(0)) continue;
-        const int64_t w = (int64_t)B.fib[k + 2];
-        TileFlip f;
-        f.k = k;
-        if (set) {
-          f.off = -w;
-          f.len = size;
-        } else {
-          if (j + 1 < n - L && ((p >> (j + 1)) & 1ULL)) continue;
-          if (j >= 1 && ((p >> (j - 1)) & 1ULL)) continue;
-          f.off = w;
-          f.len = (j == 0) ? (int)B.fib[L + 1] : size;   // k = L needs low bit L-1 clear
-        }
-        hf[cnt] = f;
-        hf_re[cnt] = are;
-        hf_im[cnt] = aim;
-        ++cnt;
-      }
-      nhf = cnt;
-      t_base = base;
-      t_size = size;
-      t_bl = bl;
-      t_delta = dp;
-    }
-    __syncthreads();
-    const int64_t base = t_base;
-    const int size = t_size;
-    const int bl = t_bl;
-    const int nh = nhf;
-    // stage the tile of x (16-byte chunks when the row segment allows it)
-    {
-      constexpr int RB = W * (int)sizeof(S);
-      if constexpr (RB > 16 && RB % 16 == 0) {
-        constexpr int NC = RB / 16;
-        const uint4 *src = reinterpret_cast<const uint4 *>(xp + (size_t)base * W);
-        uint4 *dst = reinterpret_cast<uint4 *>(xt);
-        const int nch = size * NC;
-        for (int g = threadIdx.x; g < nch; g += blockDim.x) dst[(size_t)(g % NC) * TS + g / NC] = src[g];
-      } else if constexpr (RB % 16 == 0) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(xp + (size_t)base * W);
-        uint4 *dst = reinterpret_cast<uint4 *>(xt);
-        const int nch = size * (RB / 16);
-        for (int i = threadIdx.x; i < nch; i += blockDim.x) dst[i] = src[i];
-      } else {
-        const S *src = xp + (size_t)base * W;
-        for (int i = threadIdx.x; i < size * W; i += blockDim.x) xt[i] = src[i];
-      }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < size; i += blockDim.x) {
-      const uint32_t c = lc[i];
-      S h[W];
-#pragma unroll
-      for (int q = 0; q < W; ++q) h[q] = S(0);
-      // low flips, partners in shared memory: the flippable bits are the set
-      // ones and those with both neighbours empty (bit L above the top low
-      // bit is the tile's bl); walk the set bits of that mask
-      {
-        const uint32_t lowmask = (L >= 32) ? ~0u : ((1u << L) - 1u);
-        const uint32_t occ = (c << 1) | (c >> 1) | ((uint32_t)bl << (L - 1));
-        uint32_t m = (c | (~occ & lowmask)) & s_amp;
-        while (m) {
-          const int k = __ffs(m) - 1;
-          m &= m - 1;
-          const bool set = (c >> k) & 1u;
-          const int w = s_w[k];
-          const int pi = set ? i - w : i + w;
-          const S are = s_are[k];
-          const S aim = set ? s_aim[k] : -s_aim[k];
-          S xv[W];
-          tile_ld<S, W>(xt, TS, pi, xv);
-          acc_flip<S, C, NV, RA>(h, are, aim, xv);
-        }
-      }
-      // high flips: contiguous partner rows in global memory, two in flight
-      for (int f = 0; f < nh; f += 2) {
-        S xa[W], xb[W];
-        const bool oa = i < hf[f].len;
-        const bool ob = (f + 1 < nh) && (i < hf[f + 1].len);
-        if (oa) ld_row<S, W>(xp + (size_t)(base + i + hf[f].off) * W, xa);
-        if (ob) ld_row<S, W>(xp + (size_t)(base + i + hf[f + 1].off) * W, xb);
-        if (oa) acc_flip<S, C, NV, RA>(h, hf_re[f], hf_im[f], xa);
-        if (ob) acc_flip<S, C, NV, RA>(h, hf_re[f + 1], hf_im[f + 1], xb);
-      }
-      const int64_t row = base + i;
-      S xr[W];
-      tile_ld<S, W>(xt, TS, i, xr);
-      if (!K.skip_diag) {
-        const S dsum = H.diagV[row] + t_delta + ld[i];
-#pragma unroll
-        for (int q = 0; q < W; ++q) h[q] += dsum * xr[q];
-      }
-      S yv[W];
-      const S a = (S)K.a, b = (S)K.b;
-#pragma unroll
-      for (int q = 0; q < W; ++q) yv[q] = a * h[q] + b * xr[q];
-      if (K.z) {
-        S zv[W];
-        ld_row_cs<S, W>((const S *)K.z + (size_t)row * W, zv);
-        const S cc = (S)K.c;
-#pragma unroll
-        for (int q = 0; q < W; ++q) yv[q] += cc * zv[q];
-      }
-      if (K.acc) {
-        S av[W];
-        S *ap = (S *)K.acc + (size_t)row * W;
-        ld_row_cs<S, W>(ap, av);
-        const S wr = (S)K.w_re, wi = (S)K.w_im;
-        if constexpr (C) {
-#pragma unroll
-          for (int v = 0; v < NV; ++v) {
-            av[2 * v] += wr * yv[2 * v] - wi * yv[2 * v + 1];
-            av[2 * v + 1] += wr * yv[2 * v + 1] + wi * yv[2 * v];
-          }
-        } else {
-#pragma unroll
-          for (int v = 0; v < NV; ++v) av[v] += wr * yv[v];
-        }
-        st_row_cs<S, W>(ap, av);
-      }
-      if (K.y) st_row_cs<S, W>((S *)K.y + (size_t)row * W, yv);
-      if constexpr (WANT) {
-        if constexpr (C) {
-          const double xre = xr[0], xim = xr[1], yre = yv[0], yim = yv[1];
-          q0 += xre * xre + xim * xim;
-          q1 += xre * yre + xim * yim;
-          q2 += xre * yim - xim * yre;
-          q3 += yre * yre + yim * yim;
-        } else {
-          const double xd = xr[0], yd = yv[0];
-          q0 += xd * xd;
-          q1 += xd * yd;
-          q3 += yd * yd;
-          if (K.probe) q2 += yd * (double)((const S *)K.probe)[row];
-        }
-      }
-    }
-  }
-  if constexpr (WANT) reduce4(K, q0, q1, q2, q3);
-}
-
-template <typename S>
-HamArgs<S> ham_args(const el_ham *h, const S *diagV) {
-  HamArgs<S> A;
-  memset(&A, 0, sizeof A);
-  A.diagV = diagV;
-  A.px = h->d_px;
-  A.npx = (int)h->px.size();
-  A.lossy = h->lossy ? 1 : 0;
-  A.real_amp = h->drive_complex ? 0 : 1;
-  for (int k = 0; k < h->n; ++k) {
-    A.delta[k] = (S)h->delta[k];
-    A.up_re[k] = (S)(0.5 * h->om_re[k]);
-    A.up_im[k] = (S)(0.5 * h->om_im[k]);
-    A.loss[k] = (S)h->loss[k];
-  }
-  return A;
-}
-
 int ilog2(int64_t v) {
   int l = 0;
   while ((1LL << l) < v) ++l;
@@ -1030,52 +698,88 @@ __global__ void k_gershgorin(BasisDev B, HamArgs<double> H, double *partials,
 
 // ------------------------------------------------------------ BLAS-like ops
 
-template <typename S, bool C>
-__global__ void k_axpby(int64_t len, double a_re, double a_im, const S *x,
+// y = alpha x + beta y in FP64 arithmetic and, if asked, |y|^2.  HBM-bound on
+// long vectors: 16-byte accesses (ALN: both pointers on 16-byte boundaries)
+// move 2^25 FP64 values of x, y and the result at 6.1 TB/s (4.0 with 8-byte
+// ones); on short vectors the norm's tail counts, so warps meet by shuffles
+// and the last block adds the block sums with all its threads.
+template <typename S, bool C, bool ALN>
+__global__ void __launch_bounds__(256) k_axpby(int64_t len, double a_re, double a_im, const S *x,
                         double b_re, double b_im, S *y, double *partials,
                         unsigned int *counter, double *norm2) {
-  __shared__ double red[256];
+  __shared__ double red[8];
   __shared__ bool last;
+  constexpr int E = ALN ? 16 / (int)sizeof(S) : (C ? 2 : 1);   // values per step
+  struct alignas(ALN ? 16 : sizeof(S)) Chunk { S v[E]; };
   double acc = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len;
-       i += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t values = C ? 2 * len : len;
+  // beta == 0 must not read y: workspace may hold stale bits (NaN)
+  const bool ry = (b_re != 0.0 || b_im != 0.0);
+  auto combine = [&](const S *xv, S *yv, int cnt) {
     if constexpr (C) {
-      const double xr = x ? (double)x[2 * i] : 0.0, xi = x ? (double)x[2 * i + 1] : 0.0;
-      // beta == 0 must not read y: workspace may hold stale bits (NaN)
-      const bool ry = (b_re != 0.0 || b_im != 0.0);
-      const double yr = ry ? (double)y[2 * i] : 0.0, yi = ry ? (double)y[2 * i + 1] : 0.0;
-      const double r = a_re * xr - a_im * xi + b_re * yr - b_im * yi;
-      const double im = a_re * xi + a_im * xr + b_re * yi + b_im * yr;
-      const S rs = (S)r, is = (S)im;
-      y[2 * i] = rs;
-      y[2 * i + 1] = is;
-      acc += (double)rs * (double)rs + (double)is * (double)is;
+#pragma unroll
+      for (int i = 0; i < E; i += 2) {
+        if (i >= cnt) break;
+        const double xr = xv[i], xi = xv[i + 1], yr = yv[i], yi = yv[i + 1];
+        const S rs = (S)(a_re * xr - a_im * xi + b_re * yr - b_im * yi);
+        const S is = (S)(a_re * xi + a_im * xr + b_re * yi + b_im * yr);
+        yv[i] = rs;
+        yv[i + 1] = is;
+        acc += (double)rs * (double)rs + (double)is * (double)is;
+      }
     } else {
-      const double xv = x ? (double)x[i] : 0.0;
-      const double yv = (b_re != 0.0) ? (double)y[i] : 0.0;
-      const S r = (S)(a_re * xv + b_re * yv);
-      y[i] = r;
-      acc += (double)r * (double)r;
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        if (i >= cnt) break;
+        const S r = (S)(a_re * (double)xv[i] + b_re * (double)yv[i]);
+        yv[i] = r;
+        acc += (double)r * (double)r;
+      }
     }
+  };
+  const int64_t chunks = values / E;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < chunks; c += stride) {
+    Chunk xc{}, yc{};
+    if (x) xc = reinterpret_cast<const Chunk *>(x)[c];
+    if (ry) yc = reinterpret_cast<const Chunk *>(y)[c];
+    combine(xc.v, yc.v, E);
+    reinterpret_cast<Chunk *>(y)[c] = yc;
+  }
+  const int tail = (int)(values - chunks * E);   // fewer than E values after the last chunk
+  if (tail > 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+    Chunk xc{}, yc{};
+    for (int i = 0; i < tail; ++i) {
+      if (x) xc.v[i] = x[chunks * E + i];
+      if (ry) yc.v[i] = y[chunks * E + i];
+    }
+    combine(xc.v, yc.v, tail);
+    for (int i = 0; i < tail; ++i) y[chunks * E + i] = yc.v[i];
   }
   if (!norm2) return;
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+  auto block_total = [&](double v) -> double {   // in thread 0
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-  }
+    double s = 0.0;
+    if (threadIdx.x == 0)
+      for (int w = 0; w < 8; ++w) s += red[w];
+    return s;
+  };
+  const double mine = block_total(acc);
   if (threadIdx.x == 0) {
-    partials[blockIdx.x] = red[0];
+    partials[blockIdx.x] = mine;
     __threadfence();
     last = (atomicAdd(counter, 1u) == gridDim.x - 1);
   }
   __syncthreads();
-  if (last && threadIdx.x == 0) {
-    __threadfence();
-    double s = 0.0;
-    for (unsigned i = 0; i < gridDim.x; ++i) s += __ldcg(&partials[i]);
-    *norm2 = s;
+  if (!last) return;
+  __threadfence();
+  double part = 0.0;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += 256) part += __ldcg(&partials[i]);
+  const double all = block_total(part);
+  if (threadIdx.x == 0) {
+    *norm2 = all;
     *counter = 0u;
   }
 }
@@ -1353,57 +1057,6 @@ void launch_row_t(el_ctx *ctx, int lay, int nvec, bool want, int grid, const Bas
   }
 }
 
-// Tile bits L for the chain tile kernel: the largest L whose tile (rows x
-// row bytes, plus 4 + sizeof(S) bytes of tables per row) stays within 40 KB,
-// leaving at least 4 prefix bits; 0 if the chain is too short to tile.
-int chain_tile_bits(int n, int row_bytes, int scalar_bytes) {
-  uint64_t f[70];
-  f[0] = 0; f[1] = 1;
-  for (int i = 2; i < 70; ++i) f[i] = f[i - 1] + f[i - 2];
-  int best = 0;
-  for (int L = 4; L + 4 <= n && L + 2 < 70; ++L)
-    if (f[L + 2] * (uint64_t)(row_bytes + 4 + scalar_bytes) <= 40960) best = L;
-  return best;
-}
-
-template <typename S, bool C, int NV, bool WANT, bool RA>
-int launch_chain_tile_t(el_ctx *ctx, int L, int64_t ntiles, const BasisDev &B, const HamArgs<S> &H,
-                        const KArgs &K) {
-  constexpr int W = NV * (C ? 2 : 1);
-  const size_t ts = (size_t)B.fib[L + 2];
-  const size_t smem = ts * W * sizeof(S) + ts * 4 + ts * sizeof(S) + 16;
-  cudaFuncSetAttribute(k_apply_chain_tile<S, C, NV, WANT, RA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  const int grid = (int)std::min<int64_t>(ntiles, (int64_t)sms * 8);
-  k_apply_chain_tile<S, C, NV, WANT, RA><<<grid, 256, smem, ctx->stream>>>(B, H, K, L, ntiles);
-  return EL_OK;
-}
-
-template <typename S, bool C, bool RA>
-int launch_chain_tile_r(el_ctx *ctx, int nvec, bool want, int L, int64_t ntiles, const BasisDev &B,
-                        const HamArgs<S> &H, const KArgs &K) {
-  if (want) return launch_chain_tile_t<S, C, 1, true, RA>(ctx, L, ntiles, B, H, K);
-  switch (nvec) {
-    case 1: return launch_chain_tile_t<S, C, 1, false, RA>(ctx, L, ntiles, B, H, K);
-    case 2: return launch_chain_tile_t<S, C, 2, false, RA>(ctx, L, ntiles, B, H, K);
-    case 4: return launch_chain_tile_t<S, C, 4, false, RA>(ctx, L, ntiles, B, H, K);
-    default: return launch_chain_tile_t<S, C, 8, false, RA>(ctx, L, ntiles, B, H, K);
-  }
-}
-
-// complex vectors with a real drive take the real-amplitude variant, except
-// for eight complex64 vectors per row, where it needs 119 registers instead
-// of 80 and loses the third CTA per SM
-template <typename S, bool C>
-int launch_chain_tile_v(el_ctx *ctx, int nvec, bool want, int L, int64_t ntiles, const BasisDev &B,
-                        const HamArgs<S> &H, const KArgs &K, bool real_amp) {
-  if (C && real_amp && (want || nvec <= 4 || sizeof(S) == 8))
-    return launch_chain_tile_r<S, C, true>(ctx, nvec, want, L, ntiles, B, H, K);
-  return launch_chain_tile_r<S, C, false>(ctx, nvec, want, L, ntiles, B, H, K);
-}
-
 int launch_apply_row(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const BasisDev &B, KArgs K) {
   const int lay = h->basis->layout;
   const int64_t lanes = row_lanes(B, (int)A.nvec) ? ROW_LANES : 1;
@@ -1412,28 +1065,9 @@ int launch_apply_row(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const BasisDev 
   if (want) {
     K.nvec = 1;
     K.lognv = 0;
-    // partial sums for the row grid or the tile grid (at most 8 CTAs per SM)
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    int rc = el::ensure_partials(ctx, (size_t)std::max(grid, 8 * sms) * 4);
+    int rc = el::ensure_partials(ctx, (size_t)grid * 4);
     if (rc) return rc;
     K.partials = ctx->d_partials;
-  }
-  if (lay == EL_LAYOUT_CHAIN) {
-    const int ss = (A.dtype == EL_F32 || A.dtype == EL_C64) ? 4 : 8;
-    const int L = chain_tile_bits(h->n, (int)A.nvec * el::dtype_size(A.dtype), ss);
-    if (L > 0) {
-      const int64_t ntiles = (int64_t)B.fib[h->n - L + 2];
-      switch (A.dtype) {
-        case EL_F32: launch_chain_tile_v<float, false>(ctx, A.nvec, want, L, ntiles, B, ham_args<float>(h, h->d_diagV32), K, false); break;
-        case EL_F64: launch_chain_tile_v<double, false>(ctx, A.nvec, want, L, ntiles, B, ham_args<double>(h, h->d_diagV64), K, false); break;
-        case EL_C64: launch_chain_tile_v<float, true>(ctx, A.nvec, want, L, ntiles, B, ham_args<float>(h, h->d_diagV32), K, !h->drive_complex); break;
-        case EL_C128: launch_chain_tile_v<double, true>(ctx, A.nvec, want, L, ntiles, B, ham_args<double>(h, h->d_diagV64), K, !h->drive_complex); break;
-        default: return el::fail(ctx, EL_EINVAL, "unknown dtype %d", A.dtype);
-      }
-      EL_LAUNCH_CHECK(ctx);
-      return EL_OK;
-    }
   }
   switch (A.dtype) {
     case EL_F32: launch_row_t<float, false>(ctx, lay, A.nvec, want, grid, B, ham_args<float>(h, h->d_diagV32), K); break;
@@ -1479,6 +1113,7 @@ int launch_apply(el_ctx *ctx, el_ham *h, const ApplyArgs &A) {
     int rc = ham_diag32(ctx, h);
     if (rc) return rc;
   }
+  if (chain_block_ok(h, A)) return launch_chain_block(ctx, h, A, B, K);
   if (row_kernel_ok(h, A)) return launch_apply_row(ctx, h, A, B, K);
   if (!h->px.empty() && (B.layout == EL_LAYOUT_FULL || B.layout == EL_LAYOUT_TABLE) && B.n <= 32 &&
       B.dim < ((int64_t)1 << 31)) {
@@ -1577,18 +1212,30 @@ int gershgorin(el_ctx *ctx, el_ham *h, double *lo, double *hi, double *norm1) {
 
 int launch_axpby(el_ctx *ctx, int dtype, int64_t len, double a_re, double a_im,
                  const void *x, double b_re, double b_im, void *y, double *norm2_out) {
-  const int grid = grid_for(len, 256);
+  const bool aln = (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
+  const int es = dtype_size(dtype);
+  if (!es) return fail(ctx, EL_EINVAL, "unknown dtype %d", dtype);
+  const int grid = grid_for(aln ? (len * es + 15) / 16 : len, 256);
   if (norm2_out) {
     int rc = ensure_partials(ctx, (size_t)grid);
     if (rc) return rc;
   }
+#define EL_AXPBY(S, C)                                                                                  \
+  do {                                                                                                  \
+    if (aln)                                                                                            \
+      k_axpby<S, C, true><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const S *)x, b_re, b_im,     \
+                                                         (S *)y, ctx->d_partials, ctx->d_counter, norm2_out); \
+    else                                                                                                \
+      k_axpby<S, C, false><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const S *)x, b_re, b_im,    \
+                                                          (S *)y, ctx->d_partials, ctx->d_counter, norm2_out); \
+  } while (0)
   switch (dtype) {
-    case EL_F32: k_axpby<float, false><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const float *)x, b_re, b_im, (float *)y, ctx->d_partials, ctx->d_counter, norm2_out); break;
-    case EL_F64: k_axpby<double, false><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const double *)x, b_re, b_im, (double *)y, ctx->d_partials, ctx->d_counter, norm2_out); break;
-    case EL_C64: k_axpby<float, true><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const float *)x, b_re, b_im, (float *)y, ctx->d_partials, ctx->d_counter, norm2_out); break;
-    case EL_C128: k_axpby<double, true><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const double *)x, b_re, b_im, (double *)y, ctx->d_partials, ctx->d_counter, norm2_out); break;
-    default: return fail(ctx, EL_EINVAL, "unknown dtype %d", dtype);
+    case EL_F32: EL_AXPBY(float, false); break;
+    case EL_F64: EL_AXPBY(double, false); break;
+    case EL_C64: EL_AXPBY(float, true); break;
+    default: EL_AXPBY(double, true); break;
   }
+#undef EL_AXPBY
   EL_LAUNCH_CHECK(ctx);
   return EL_OK;
 }
