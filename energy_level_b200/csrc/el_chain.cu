@@ -195,10 +195,41 @@ __device__ __forceinline__ void store_cs(Chunk<S, CW> *p, const Chunk<S, CW> &c)
   else __stcs(reinterpret_cast<unsigned *>(p), u.w);
 }
 
+// out[o] = sum of rows[b][o] over b < nrows, in a fixed order, by the whole
+// block: output o by nt / nout threads, each adding every (nt / nout)-th row.
+__device__ __forceinline__ void sum_rows(const double *rows, int nrows, int nout, double *sm, double *out,
+                                         int odst, int osrc) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int per = nout <= nt ? nt / nout : 1;
+  for (int o0 = 0; o0 < nout; o0 += nt) {
+    const int o = o0 + (per > 1 ? tid % nout : tid), sh = per > 1 ? tid / nout : 0;
+    const bool on = o < nout && sh < per;
+    double s = 0.0;
+    if (on) {
+#pragma unroll 8
+      for (int b = sh; b < nrows; b += per) s += __ldcg(&rows[(size_t)b * nout + o]);
+    }
+    __syncthreads();
+    if (per > 1) {
+      if (on) sm[sh * nout + o] = s;
+      __syncthreads();
+      if (on && sh == 0) {
+        s = 0.0;
+        for (int w = 0; w < per; ++w) s += sm[w * nout + o];
+      }
+    }
+    if (on && sh == 0) out[(o / osrc) * odst + o % osrc] = s;
+  }
+}
+
 // Sums of the dot products over the launch: lanes of a warp that hold the
-// same chunk of a row meet by shuffles, warps in shared memory, blocks in
-// global memory, where the last block to finish adds them in a fixed order.
-// q: 4 values (xx, Re xy, Im xy or <y, probe>, yy) per vector of the chunk.
+// same chunk of a row meet by shuffles, warps in shared memory, and blocks in
+// global memory in two levels: the last block of each group of `group` to
+// finish adds its group's sums, the last group's the groups' (all in fixed
+// orders).  One level, the very last block adding 592 rows of 128 sums,
+// took 130 of the 160 us of a step with 32 vectors on 24 sites.
+// q: ND values (xx, Re xy, then Im xy or <y, probe>, yy) per vector of the chunk.
+constexpr int DOT_GROUPS = 48;      // counters 1 .. DOT_GROUPS of the context
 template <int CV, int ND>
 __device__ void block_dots(const KArgs &K, int nch, double (&q)[CV][ND], double *sm) {
   __shared__ bool last;
@@ -210,12 +241,12 @@ __device__ void block_dots(const KArgs &K, int nch, double (&q)[CV][ND], double 
     for (int c = 0; c < ND; ++c)
       for (int o = 16; o >= nch; o >>= 1) q[v][c] += __shfl_xor_sync(0xffffffffu, q[v][c], o);
   __syncthreads();                    // the tile in shared memory is done with
-  const int nout = nch * CV * 4;      // = nvec * 4, in the order of K.dots
+  const int nout = nch * CV * ND;
   if (lane < nch) {
 #pragma unroll
     for (int v = 0; v < CV; ++v)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) sm[warp * nout + (lane * CV + v) * 4 + c] = c < ND ? q[v][c < ND ? c : 0] : 0.0;
+      for (int c = 0; c < ND; ++c) sm[warp * nout + (lane * CV + v) * ND + c] = q[v][c];
   }
   __syncthreads();
   for (int o = tid; o < nout; o += nt) {
@@ -223,34 +254,27 @@ __device__ void block_dots(const KArgs &K, int nch, double (&q)[CV][ND], double 
     for (int w = 0; w < nw; ++w) s += sm[w * nout + o];
     K.partials[(size_t)blockIdx.x * nout + o] = s;
   }
+  const int nb = (int)gridDim.x;
+  const int group = max(16, (nb + DOT_GROUPS - 1) / DOT_GROUPS);
+  const int ngroups = (nb + group - 1) / group, g = (int)blockIdx.x / group;
+  const int first = g * group, size = min(group, nb - first);
+  double *gsum = K.partials + (size_t)nb * nout;
   __threadfence();
   __syncthreads();
-  if (tid == 0) last = (atomicAdd(K.counter, 1u) == gridDim.x - 1);
+  if (tid == 0) last = (atomicAdd(&K.counter[1 + g], 1u) == (unsigned)size - 1);
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // shares of blocks per output: thread = share * nout + output
-  const int per = nout <= nt ? nt / nout : 1;
-  for (int o0 = 0; o0 < nout; o0 += nt) {
-    const int o = o0 + (per > 1 ? tid % nout : tid), sh = per > 1 ? tid / nout : 0;
-    const bool on = o < nout && sh < per;
-    double s = 0.0;
-    if (on) {
-#pragma unroll 8
-      for (unsigned b = sh; b < gridDim.x; b += per) s += __ldcg(&K.partials[(size_t)b * nout + o]);
-    }
-    if (per > 1) {
-      __syncthreads();
-      if (on) sm[sh * nout + o] = s;
-      __syncthreads();
-      if (on && sh == 0) {
-        s = 0.0;
-        for (int w = 0; w < per; ++w) s += sm[w * nout + o];
-      }
-    }
-    if (on && sh == 0) K.dots[o] = s;
-  }
-  if (tid == 0) *K.counter = 0u;
+  sum_rows(K.partials + (size_t)first * nout, size, nout, sm, gsum + (size_t)g * nout, 1, 1);
+  if (tid == 0) K.counter[1 + g] = 0u;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) last = (atomicAdd(&K.counter[0], 1u) == (unsigned)ngroups - 1);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  sum_rows(gsum, ngroups, nout, sm, K.dots, 4, ND);
+  if (tid == 0) K.counter[0] = 0u;
 }
 
 // One tile: the NS sub-blocks of the thread's low code.  Threads without a
@@ -558,7 +582,7 @@ int launch_block_t(el_ctx *ctx, const ChainGeom &G, const HamArgs<S> &H, KArgs K
   const int64_t ntiles = G.tiles[0] + G.tiles[1];
   const int grid = (int)std::min<int64_t>(ntiles, (int64_t)sms * std::max(per_sm, 1));
   if (ND) {
-    const int rc = ensure_partials(ctx, (size_t)grid * nout);
+    const int rc = ensure_partials(ctx, (size_t)(grid + DOT_GROUPS) * nout);
     if (rc) return rc;
     K.partials = ctx->d_partials;
   }
