@@ -80,6 +80,26 @@ def product_vectors(spec, n):
     return _product_sites(spec, int(n))
 
 
+def basis_code(spec, n):
+    """The code of a product of exactly |g> and |r> on every site (amplitude
+    1), or None for any other spec."""
+    n = int(n)
+    if _form(spec, n) != 'product':
+        return None
+    sites = _product_sites(spec, n)
+    if sites is None:
+        return None
+    code = 0
+    for loc in sites:
+        if loc[0] == 1.0 and loc[1] == 0.0:
+            code <<= 1
+        elif loc[0] == 0.0 and loc[1] == 1.0:
+            code = (code << 1) | 1
+        else:
+            return None
+    return code
+
+
 # grammar forms, tested in this order (the first match decides)
 def _looks_full_list(spec, n):
     return (isinstance(spec, (list, tuple)) and len(spec) == (1 << n)
