@@ -1,6 +1,8 @@
-// Generic fused H-apply kernel and the vector helpers used by the drivers.
+// Generic fused H-apply kernel, the row kernel of small bases and the vector
+// helpers used by the drivers (large chain, ring and full bases: el_chain.cu,
+// el_full.cu).
 //
-// One thread handles one (row, vector) element of a block [dim][nvec]; the
+// Generic: one thread handles one (row, vector) element of a block [dim][nvec]; the
 // nvec lanes of a row are adjacent, so every flip gather of a row block is a
 // contiguous nvec-element segment.  For each row the kernel
 //   - recovers the configuration code (arithmetic unranking or code table),
@@ -328,26 +330,13 @@ __global__ void __launch_bounds__(256) k_apply_hop(BasisDev B, HamArgs<S> H, KAr
 }
 
 // ------------------------------------------------- row kernel (FULL/CHAIN/RING)
-// One thread per row and all NV vectors of that row (NV <= 8): the code of a
-// row is recovered once and every flip gather moves the row's whole NV-vector
-// segment with 16-byte loads.  The bit loop runs over k = 0..n-1 in the same
-// order in every thread (warp-uniform k), so Fibonacci weights, amplitudes
-// and detunings are broadcast kernel-parameter reads; a flip that leaves the
-// basis only predicates its load off.  Four bits per round (eight per lane
-// when G lanes share a row, below) issue their gathers before any of them
-// is accumulated.  CT/RT are 32-bit when the
-// code has at most 32 bits and the basis fewer than 2^31 rows, which halves
-// the integer work of unranking and target arithmetic.
-//
-// G > 1 (single vector, small bases): G adjacent lanes of a warp share one
-// row and take the bits k = lane, lane + G, ...; their partial flip sums and
-// detunings meet in a butterfly of warp shuffles and the row's first lane
-// runs the epilogue.  A basis of a few ten thousand rows fills only part of
-// the 148 SMs with one thread per row, and each thread then waits for n
-// dependent rounds of gathers; G lanes per row cut that chain by G and give
-// the grid G times more warps.  The row loop is uniform over the block so
-// that every lane reaches the shuffles; lanes past the last row work on
-// row 0 and store nothing.
+// One vector on a small basis: G adjacent lanes of a warp share one row and
+// take the bits k = lane, lane + G, ...; eight bits per round (a lane issues
+// their gathers before it adds any of them), codes, ranks and targets in 32
+// bits.  The lanes' flip sums and detunings meet in a butterfly of shuffles
+// and the row's first lane runs the epilogue.  The row loop is uniform over
+// the block so that every lane reaches the shuffles; lanes past the last row
+// work on row 0 and store nothing.
 
 template <typename S, int W>
 __device__ __forceinline__ void ld_row(const S *p, S (&v)[W]) {
@@ -439,11 +428,14 @@ __device__ __forceinline__ RT ring_rank_t(const BasisDev &B, CT c, int n) {
   return r;
 }
 
-template <typename S, bool C, int NV, int LAY, bool WANT, typename CT, typename RT, int G>
+template <typename S, bool C, int LAY, bool WANT, int G>
 __global__ void __launch_bounds__(256) k_apply_row(BasisDev B, HamArgs<S> H, KArgs K) {
-  static_assert(G == 1 || (NV == 1 && 32 % G == 0), "lanes per row: G divides 32, one vector");
-  constexpr int W = NV * (C ? 2 : 1);
-  constexpr int U = G == 1 ? 4 : 8;   // with lanes, one round covers up to 8 G sites
+  static_assert(32 % G == 0, "lanes per row: G divides 32");
+  typedef uint32_t CT;
+  typedef int32_t RT;
+  constexpr int NV = 1;
+  constexpr int W = C ? 2 : 1;
+  constexpr int U = 8;   // one round covers 8 G sites
   const int n = B.n;
   const CT full = (n >= (int)(8 * sizeof(CT))) ? ~(CT)0 : (((CT)1 << n) - 1);
   const S *__restrict__ xp = (const S *)K.x;
@@ -455,9 +447,6 @@ __global__ void __launch_bounds__(256) k_apply_row(BasisDev B, HamArgs<S> H, KAr
   for (RT base = (RT)blockIdx.x * rpb; base < dim; base += stride) {
     const RT mine = base + (RT)(threadIdx.x / G);
     const bool active = mine < dim;       // the same for the G lanes of a row
-    if constexpr (G == 1) {
-      if (!active) break;
-    }
     const RT row = active ? mine : (RT)0;
     const CT code = unrank_fib<LAY, CT, RT>(B, row);
     CT allowed = full;
@@ -526,15 +515,13 @@ __global__ void __launch_bounds__(256) k_apply_row(BasisDev B, HamArgs<S> H, KAr
         }
       }
     }
-    if constexpr (G > 1) {
 #pragma unroll
-      for (int off = G / 2; off > 0; off >>= 1) {
+    for (int off = G / 2; off > 0; off >>= 1) {
 #pragma unroll
-        for (int i = 0; i < W; ++i) h[i] += __shfl_xor_sync(0xffffffffu, h[i], off);
-        dsum += __shfl_xor_sync(0xffffffffu, dsum, off);
-      }
-      if (lane != 0 || !active) continue;
+      for (int i = 0; i < W; ++i) h[i] += __shfl_xor_sync(0xffffffffu, h[i], off);
+      dsum += __shfl_xor_sync(0xffffffffu, dsum, off);
     }
+    if (lane != 0 || !active) continue;
     S xr[W];
     ld_row<S, W>(xp + (size_t)row * W, xr);
     if (!K.skip_diag) {
@@ -996,71 +983,45 @@ bool is_complex(int dtype) { return dtype == EL_C64 || dtype == EL_C128; }
 
 namespace {
 
-// The row kernel serves FULL/CHAIN/RING bases with 1..8 vectors per row
-// (dot products only for one vector) when every vector pointer is aligned for
-// its row-segment loads.
+// Rows below which one vector goes to the row kernel: a launch is then all
+// latency, and the row kernel's chain (its gathers) is shorter than the tiled
+// kernels' (tile, barrier, gathers).  Full basis, complex128: n = 14 4.5
+// against 6.3 us, 15 6.2 against 6.5, 16 10.3 against 7.2.  Chains, float64:
+// n = 18 4.7 against 8.3, 22 8.3 against 10.3, 23 (75,025 rows) 10.3 both.
+constexpr int64_t ROW_FULL = 1 << 16, ROW_SECTOR = 148 * 512;
+constexpr int ROW_LANES = 4;
+
 bool row_kernel_ok(const el_ham *h, const ApplyArgs &A) {
   if (!h->px.empty() || h->lossy) return false;   // exchange channels or loss: generic kernel
   const int lay = h->basis->layout;
   if (lay != EL_LAYOUT_FULL && lay != EL_LAYOUT_CHAIN && lay != EL_LAYOUT_RING) return false;
-  if (A.nvec > 8) return false;
-  if (A.dots && A.nvec != 1) return false;
-  const size_t row_bytes = (size_t)A.nvec * el::dtype_size(A.dtype);
-  const size_t align = row_bytes >= 16 ? 16 : row_bytes;
+  if (A.nvec != 1 || h->n > 32 || h->basis->dim >= (lay == EL_LAYOUT_FULL ? ROW_FULL : ROW_SECTOR)) return false;
+  const size_t align = dtype_size(A.dtype);
   for (const void *p : {A.x, (const void *)A.z, (const void *)A.y, (const void *)A.acc, A.probe})
     if (p && ((uintptr_t)p % align) != 0) return false;
   return true;
 }
 
-template <typename S, bool C, int NV, bool WANT, typename CT, typename RT, int G>
-void launch_row_ct(el_ctx *ctx, int lay, int grid, const BasisDev &B, const HamArgs<S> &H, const KArgs &K) {
-  if (lay == EL_LAYOUT_FULL)
-    k_apply_row<S, C, NV, EL_LAYOUT_FULL, WANT, CT, RT, G><<<grid, 256, 0, ctx->stream>>>(B, H, K);
-  else if (lay == EL_LAYOUT_CHAIN)
-    k_apply_row<S, C, NV, EL_LAYOUT_CHAIN, WANT, CT, RT, G><<<grid, 256, 0, ctx->stream>>>(B, H, K);
-  else
-    k_apply_row<S, C, NV, EL_LAYOUT_RING, WANT, CT, RT, G><<<grid, 256, 0, ctx->stream>>>(B, H, K);
-}
-
-// Rows below which a single-vector row kernel gives each row ROW_LANES lanes:
-// one thread per row would occupy fewer than two CTAs of 256 per SM.
-constexpr int64_t LANE_ROWS = 148 * 512;
-constexpr int ROW_LANES = 4;
-
-bool row_lanes(const BasisDev &B, int nvec) {
-  return nvec == 1 && B.n <= 32 && B.dim < LANE_ROWS;
-}
-
-template <typename S, bool C, int NV, bool WANT>
+template <typename S, bool C, bool WANT>
 void launch_row_lay(el_ctx *ctx, int lay, int grid, const BasisDev &B, const HamArgs<S> &H, const KArgs &K) {
-  if constexpr (NV == 1) {
-    if (row_lanes(B, NV)) {
-      launch_row_ct<S, C, NV, WANT, uint32_t, int32_t, ROW_LANES>(ctx, lay, grid, B, H, K);
-      return;
-    }
-  }
-  if (B.n <= 32 && B.dim < ((int64_t)1 << 31))
-    launch_row_ct<S, C, NV, WANT, uint32_t, int32_t, 1>(ctx, lay, grid, B, H, K);
+  if (lay == EL_LAYOUT_FULL)
+    k_apply_row<S, C, EL_LAYOUT_FULL, WANT, ROW_LANES><<<grid, 256, 0, ctx->stream>>>(B, H, K);
+  else if (lay == EL_LAYOUT_CHAIN)
+    k_apply_row<S, C, EL_LAYOUT_CHAIN, WANT, ROW_LANES><<<grid, 256, 0, ctx->stream>>>(B, H, K);
   else
-    launch_row_ct<S, C, NV, WANT, uint64_t, int64_t, 1>(ctx, lay, grid, B, H, K);
+    k_apply_row<S, C, EL_LAYOUT_RING, WANT, ROW_LANES><<<grid, 256, 0, ctx->stream>>>(B, H, K);
 }
 
 template <typename S, bool C>
-void launch_row_t(el_ctx *ctx, int lay, int nvec, bool want, int grid, const BasisDev &B,
-                  const HamArgs<S> &H, const KArgs &K) {
-  if (want) { launch_row_lay<S, C, 1, true>(ctx, lay, grid, B, H, K); return; }
-  switch (nvec) {
-    case 1: launch_row_lay<S, C, 1, false>(ctx, lay, grid, B, H, K); break;
-    case 2: launch_row_lay<S, C, 2, false>(ctx, lay, grid, B, H, K); break;
-    case 4: launch_row_lay<S, C, 4, false>(ctx, lay, grid, B, H, K); break;
-    default: launch_row_lay<S, C, 8, false>(ctx, lay, grid, B, H, K); break;
-  }
+void launch_row_t(el_ctx *ctx, int lay, bool want, int grid, const BasisDev &B, const HamArgs<S> &H,
+                  const KArgs &K) {
+  if (want) launch_row_lay<S, C, true>(ctx, lay, grid, B, H, K);
+  else launch_row_lay<S, C, false>(ctx, lay, grid, B, H, K);
 }
 
 int launch_apply_row(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const BasisDev &B, KArgs K) {
   const int lay = h->basis->layout;
-  const int64_t lanes = row_lanes(B, (int)A.nvec) ? ROW_LANES : 1;
-  const int grid = el::grid_for(h->basis->dim * lanes, 256);
+  const int grid = el::grid_for(h->basis->dim * ROW_LANES, 256);
   const bool want = K.want != 0;
   if (want) {
     K.nvec = 1;
@@ -1070,10 +1031,10 @@ int launch_apply_row(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const BasisDev 
     K.partials = ctx->d_partials;
   }
   switch (A.dtype) {
-    case EL_F32: launch_row_t<float, false>(ctx, lay, A.nvec, want, grid, B, ham_args<float>(h, h->d_diagV32), K); break;
-    case EL_F64: launch_row_t<double, false>(ctx, lay, A.nvec, want, grid, B, ham_args<double>(h, h->d_diagV64), K); break;
-    case EL_C64: launch_row_t<float, true>(ctx, lay, A.nvec, want, grid, B, ham_args<float>(h, h->d_diagV32), K); break;
-    case EL_C128: launch_row_t<double, true>(ctx, lay, A.nvec, want, grid, B, ham_args<double>(h, h->d_diagV64), K); break;
+    case EL_F32: launch_row_t<float, false>(ctx, lay, want, grid, B, ham_args<float>(h, h->d_diagV32), K); break;
+    case EL_F64: launch_row_t<double, false>(ctx, lay, want, grid, B, ham_args<double>(h, h->d_diagV64), K); break;
+    case EL_C64: launch_row_t<float, true>(ctx, lay, want, grid, B, ham_args<float>(h, h->d_diagV32), K); break;
+    case EL_C128: launch_row_t<double, true>(ctx, lay, want, grid, B, ham_args<double>(h, h->d_diagV64), K); break;
     default: return el::fail(ctx, EL_EINVAL, "unknown dtype %d", A.dtype);
   }
   EL_LAUNCH_CHECK(ctx);
@@ -1113,8 +1074,9 @@ int launch_apply(el_ctx *ctx, el_ham *h, const ApplyArgs &A) {
     int rc = ham_diag32(ctx, h);
     if (rc) return rc;
   }
-  if (chain_block_ok(h, A)) return launch_chain_block(ctx, h, A, B, K);
   if (row_kernel_ok(h, A)) return launch_apply_row(ctx, h, A, B, K);
+  if (chain_block_ok(h, A)) return launch_chain_block(ctx, h, A, B, K);
+  if (full_block_ok(h, A)) return launch_full_block(ctx, h, A, K);
   if (!h->px.empty() && (B.layout == EL_LAYOUT_FULL || B.layout == EL_LAYOUT_TABLE) && B.n <= 32 &&
       B.dim < ((int64_t)1 << 31)) {
     const size_t sm = (size_t)B.n * B.n * (single ? sizeof(float) : sizeof(double)) * 2;

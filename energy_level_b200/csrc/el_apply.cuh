@@ -56,4 +56,8 @@ inline HamArgs<S> ham_args(const el_ham *h, const S *diagV) {
 bool chain_block_ok(const el_ham *h, const ApplyArgs &A);
 int launch_chain_block(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const BasisDev &B, const KArgs &K);
 
+// The same on the full 2^n basis (el_full.cu).
+bool full_block_ok(const el_ham *h, const ApplyArgs &A);
+int launch_full_block(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const KArgs &K);
+
 }  // namespace el

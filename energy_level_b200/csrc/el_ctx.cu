@@ -112,6 +112,7 @@ int el_ctx_create(int device, void *stream, el_ctx **out) {
   ctx->device = device;
   ctx->stream = (cudaStream_t)stream;
   if (cudaSetDevice(device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
       cudaMalloc(&ctx->d_counter, 64 * sizeof(unsigned int)) != cudaSuccess ||
       cudaMemset(ctx->d_counter, 0, 64 * sizeof(unsigned int)) != cudaSuccess ||
       cudaMalloc(&ctx->d_scalars, EL_SCALARS * sizeof(double)) != cudaSuccess ||

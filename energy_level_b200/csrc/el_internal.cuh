@@ -27,6 +27,7 @@
 
 struct el_ctx {
   int device = 0;
+  int sms = 148;           // multiprocessors of the device
   cudaStream_t stream = nullptr;
   std::string err;
   const volatile int32_t *cancel = nullptr;
@@ -133,6 +134,7 @@ BasisDev basis_dev(const el_basis *b);
 int ham_diag32(el_ctx *ctx, el_ham *h);
 int dtype_size(int dtype);
 int grid_for(int64_t work, int block);
+inline int sm_count(const el_ctx *ctx) { return ctx->sms; }
 // Cached device workspace `slot` of at least `bytes` bytes (nullptr on failure,
 // with the error recorded on ctx).
 void *workspace(el_ctx *ctx, int slot, size_t bytes);
