@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(256) k_apply(BasisDev B, HamArgs<S> H, KArgs K
     if constexpr (C) {
       yv.re = (S)K.a * hre + (S)K.b * xr.re;
       yv.im = (S)K.a * him + (S)K.b * xr.im;
-      if (K.z) { const V zv = V::load(K.z, t); yv.re += (S)K.c * zv.re; yv.im += (S)K.c * zv.im; }
+      if (K.z) { const V zv = V::load(K.z, t); yv.re += (S)coef_c(K) * zv.re; yv.im += (S)coef_c(K) * zv.im; }
       if (K.acc) {
         V av = V::load(K.acc, t);
         av.re += (S)K.w_re * yv.re - (S)K.w_im * yv.im;
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256) k_apply(BasisDev B, HamArgs<S> H, KArgs K
       }
     } else {
       yv.v = (S)K.a * hre + (S)K.b * xr.v;
-      if (K.z) { const V zv = V::load(K.z, t); yv.v += (S)K.c * zv.v; }
+      if (K.z) { const V zv = V::load(K.z, t); yv.v += (S)coef_c(K) * zv.v; }
       if (K.acc) { V av = V::load(K.acc, t); av.v += (S)K.w_re * yv.v; av.store(K.acc, t); }
     }
     if (K.y) yv.store(K.y, t);
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(256) k_apply_hop(BasisDev B, HamArgs<S> H, KAr
     if constexpr (C) {
       yv.re = (S)K.a * hre + (S)K.b * xr.re;
       yv.im = (S)K.a * him + (S)K.b * xr.im;
-      if (K.z) { const V zv = V::load(K.z, t); yv.re += (S)K.c * zv.re; yv.im += (S)K.c * zv.im; }
+      if (K.z) { const V zv = V::load(K.z, t); yv.re += (S)coef_c(K) * zv.re; yv.im += (S)coef_c(K) * zv.im; }
       if (K.acc) {
         V av = V::load(K.acc, t);
         av.re += (S)K.w_re * yv.re - (S)K.w_im * yv.im;
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(256) k_apply_hop(BasisDev B, HamArgs<S> H, KAr
       }
     } else {
       yv.v = (S)K.a * hre + (S)K.b * xr.v;
-      if (K.z) { const V zv = V::load(K.z, t); yv.v += (S)K.c * zv.v; }
+      if (K.z) { const V zv = V::load(K.z, t); yv.v += (S)coef_c(K) * zv.v; }
       if (K.acc) { V av = V::load(K.acc, t); av.v += (S)K.w_re * yv.v; av.store(K.acc, t); }
     }
     if (K.y) yv.store(K.y, t);
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(256) k_apply_row(BasisDev B, HamArgs<S> H, KAr
     if (K.z) {
       S zv[W];
       ld_row<S, W>((const S *)K.z + (size_t)row * W, zv);
-      const S c = (S)K.c;
+      const S c = (S)coef_c(K);
 #pragma unroll
       for (int i = 0; i < W; ++i) yv[i] += c * zv[i];
     }
@@ -685,6 +685,12 @@ __global__ void k_gershgorin(BasisDev B, HamArgs<double> H, double *partials,
 
 // ------------------------------------------------------------ BLAS-like ops
 
+// Scalars of launch_lanczos_update (dots null: a plain axpby).
+struct LanczosScalars {
+  const double *dots, *k2;
+  double *rec;
+};
+
 // y = alpha x + beta y in FP64 arithmetic and, if asked, |y|^2.  HBM-bound on
 // long vectors: 16-byte accesses (ALN: both pointers on 16-byte boundaries)
 // move 2^25 FP64 values of x, y and the result at 6.1 TB/s (4.0 with 8-byte
@@ -693,12 +699,25 @@ __global__ void k_gershgorin(BasisDev B, HamArgs<double> H, double *partials,
 template <typename S, bool C, bool ALN>
 __global__ void __launch_bounds__(256) k_axpby(int64_t len, double a_re, double a_im, const S *x,
                         double b_re, double b_im, S *y, double *partials,
-                        unsigned int *counter, double *norm2) {
+                        unsigned int *counter, double *norm2, LanczosScalars U) {
   __shared__ double red[8];
   __shared__ bool last;
   constexpr int E = ALN ? 16 / (int)sizeof(S) : (C ? 2 : 1);   // values per step
   struct alignas(ALN ? 16 : sizeof(S)) Chunk { S v[E]; };
-  double acc = 0.0;
+  double acc = 0.0, alpha = 0.0, bpred = 1.0, k2 = 1.0;
+  if (U.dots) {
+    k2 = U.k2 ? *U.k2 : 1.0;
+    alpha = U.dots[1] / k2;
+    double sc = 1.0;
+    if (U.k2) {
+      // |w - alpha v|^2 from <y, y>; where that cancels, the norm is formed directly
+      const double bp2 = U.dots[3] / k2 - alpha * alpha, s1 = fmax(1.0, fabs(alpha));
+      bpred = bp2 > 1e-6 * s1 * s1 ? sqrt(bp2) : 1.0;
+      sc = 1.0 / (sqrt(k2) * bpred);
+    }
+    a_re = -alpha * sc;
+    b_re = sc;
+  }
   const int64_t values = C ? 2 * len : len;
   // beta == 0 must not read y: workspace may hold stale bits (NaN)
   const bool ry = (b_re != 0.0 || b_im != 0.0);
@@ -743,7 +762,7 @@ __global__ void __launch_bounds__(256) k_axpby(int64_t len, double a_re, double 
     combine(xc.v, yc.v, tail);
     for (int i = 0; i < tail; ++i) y[chunks * E + i] = yc.v[i];
   }
-  if (!norm2) return;
+  if (!norm2 && !U.dots) return;
   auto block_total = [&](double v) -> double {   // in thread 0
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
@@ -766,7 +785,15 @@ __global__ void __launch_bounds__(256) k_axpby(int64_t len, double a_re, double 
   for (unsigned i = threadIdx.x; i < gridDim.x; i += 256) part += __ldcg(&partials[i]);
   const double all = block_total(part);
   if (threadIdx.x == 0) {
-    *norm2 = all;
+    if (U.dots) {
+      U.rec[0] = alpha;
+      U.rec[1] = all;
+      U.rec[2] = -sqrt(all) * bpred * sqrt(all) / sqrt(k2);
+      if (!U.k2) U.rec[2] = -sqrt(all);
+      U.rec[3] = bpred;
+    } else {
+      *norm2 = all;
+    }
     *counter = 0u;
   }
 }
@@ -1056,7 +1083,7 @@ int launch_apply(el_ctx *ctx, el_ham *h, const ApplyArgs &A) {
   K.nvec = nvec;
   K.lognv = ilog2(nvec);
   K.x = A.x; K.z = A.z; K.y = A.y; K.acc = A.acc;
-  K.a = A.a; K.b = A.b; K.c = A.c; K.w_re = A.w_re; K.w_im = A.w_im;
+  K.a = A.a; K.b = A.b; K.c = A.c; K.c_dev = A.c_dev; K.w_re = A.w_re; K.w_im = A.w_im;
   K.dots = A.dots;
   K.want = A.dots ? (A.want_dots ? A.want_dots : 7) : 0;
   K.skip_diag = A.skip_diag;
@@ -1172,24 +1199,26 @@ int gershgorin(el_ctx *ctx, el_ham *h, double *lo, double *hi, double *norm1) {
   return EL_OK;
 }
 
-int launch_axpby(el_ctx *ctx, int dtype, int64_t len, double a_re, double a_im,
-                 const void *x, double b_re, double b_im, void *y, double *norm2_out) {
+static int axpby(el_ctx *ctx, int dtype, int64_t len, double a_re, double a_im, const void *x, double b_re,
+                 double b_im, void *y, double *norm2_out, const LanczosScalars &U) {
   const bool aln = (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
   const int es = dtype_size(dtype);
   if (!es) return fail(ctx, EL_EINVAL, "unknown dtype %d", dtype);
   const int grid = grid_for(aln ? (len * es + 15) / 16 : len, 256);
-  if (norm2_out) {
+  if (norm2_out || U.dots) {
     int rc = ensure_partials(ctx, (size_t)grid);
     if (rc) return rc;
   }
-#define EL_AXPBY(S, C)                                                                                  \
-  do {                                                                                                  \
-    if (aln)                                                                                            \
-      k_axpby<S, C, true><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const S *)x, b_re, b_im,     \
-                                                         (S *)y, ctx->d_partials, ctx->d_counter, norm2_out); \
-    else                                                                                                \
-      k_axpby<S, C, false><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const S *)x, b_re, b_im,    \
-                                                          (S *)y, ctx->d_partials, ctx->d_counter, norm2_out); \
+#define EL_AXPBY(S, C)                                                                                 \
+  do {                                                                                                 \
+    if (aln)                                                                                           \
+      k_axpby<S, C, true><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const S *)x, b_re, b_im,    \
+                                                         (S *)y, ctx->d_partials, ctx->d_counter,      \
+                                                         norm2_out, U);                                \
+    else                                                                                               \
+      k_axpby<S, C, false><<<grid, 256, 0, ctx->stream>>>(len, a_re, a_im, (const S *)x, b_re, b_im,   \
+                                                          (S *)y, ctx->d_partials, ctx->d_counter,     \
+                                                          norm2_out, U);                               \
   } while (0)
   switch (dtype) {
     case EL_F32: EL_AXPBY(float, false); break;
@@ -1200,6 +1229,16 @@ int launch_axpby(el_ctx *ctx, int dtype, int64_t len, double a_re, double a_im,
 #undef EL_AXPBY
   EL_LAUNCH_CHECK(ctx);
   return EL_OK;
+}
+
+int launch_axpby(el_ctx *ctx, int dtype, int64_t len, double a_re, double a_im,
+                 const void *x, double b_re, double b_im, void *y, double *norm2_out) {
+  return axpby(ctx, dtype, len, a_re, a_im, x, b_re, b_im, y, norm2_out, LanczosScalars{nullptr, nullptr, nullptr});
+}
+
+int launch_lanczos_update(el_ctx *ctx, int dtype, int64_t len, const void *x, void *y, const double *dots,
+                          const double *k2, double *rec) {
+  return axpby(ctx, dtype, len, 0, 0, x, 1, 0, y, nullptr, LanczosScalars{dots, k2, rec});
 }
 
 int launch_gemv_t(el_ctx *ctx, int dtype, int64_t len, int k, const void *V,

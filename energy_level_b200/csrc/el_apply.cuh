@@ -26,6 +26,7 @@ struct KArgs {
   void *y;
   void *acc;
   double a, b, c, w_re, w_im;
+  const double *c_dev;    // if not null: c from the device (written by an earlier launch)
   double *dots;
   int want;
   int skip_diag;
@@ -33,6 +34,8 @@ struct KArgs {
   double *partials;
   unsigned int *counter;
 };
+
+__device__ __forceinline__ double coef_c(const KArgs &K) { return K.c_dev ? *K.c_dev : K.c; }
 
 template <typename S>
 inline HamArgs<S> ham_args(const el_ham *h, const S *diagV) {

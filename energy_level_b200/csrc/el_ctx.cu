@@ -56,7 +56,7 @@ int grid_for(int64_t work, int block) {
 }
 
 void *workspace(el_ctx *ctx, int slot, size_t bytes) {
-  if (slot < 0 || slot >= 16) { fail(ctx, EL_EINVAL, "bad workspace slot"); return nullptr; }
+  if (slot < 0 || slot >= EL_WORKSPACES) { fail(ctx, EL_EINVAL, "bad workspace slot"); return nullptr; }
   if (bytes == 0) bytes = 16;
   if (ctx->ws_size[slot] >= bytes) return ctx->ws_ptr[slot];
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
@@ -131,7 +131,7 @@ int el_ctx_destroy(el_ctx *ctx) {
   if (ctx->d_counter) cudaFree(ctx->d_counter);
   if (ctx->d_scalars) cudaFree(ctx->d_scalars);
   if (ctx->h_scalars) cudaFreeHost(ctx->h_scalars);
-  for (int i = 0; i < 16; ++i) if (ctx->ws_ptr[i]) cudaFree(ctx->ws_ptr[i]);
+  for (int i = 0; i < EL_WORKSPACES; ++i) if (ctx->ws_ptr[i]) cudaFree(ctx->ws_ptr[i]);
   delete ctx;
   return EL_OK;
 }

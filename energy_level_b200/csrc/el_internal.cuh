@@ -24,6 +24,7 @@
 #include "../../include/energy_level_b200.h"
 
 #define EL_MAX_SITES 64
+#define EL_WORKSPACES 20
 
 struct el_ctx {
   int device = 0;
@@ -42,8 +43,8 @@ struct el_ctx {
   double *d_scalars = nullptr;   // EL_SCALARS doubles
   double *h_scalars = nullptr;   // pinned
   // cached device workspace slots (grown on demand, freed with the context)
-  void *ws_ptr[16] = {nullptr};
-  size_t ws_size[16] = {0};
+  void *ws_ptr[EL_WORKSPACES] = {nullptr};
+  size_t ws_size[EL_WORKSPACES] = {0};
   int adjoint_mode = 0;    // EL_ADJ_*: how el_adjoint_pulse schedules its sweeps
 };
 #define EL_SCALARS 4096
@@ -307,6 +308,7 @@ struct ApplyArgs {
   void *y;             // may be null (only dots/acc wanted)
   void *acc;           // may be null
   double a, b, c;
+  const double *c_dev; // if not null: c is read on the device when the launch runs
   double w_re, w_im;   // acc coefficient
   double *dots;        // device [nvec*4] or null
   int want_dots;       // bitmask: 1 xx, 2 xy, 4 yy
@@ -327,6 +329,14 @@ int gershgorin(el_ctx *ctx, el_ham *h, double *lo, double *hi, double *norm1 = n
 int launch_axpby(el_ctx *ctx, int dtype, int64_t len, double a_re, double a_im,
                  const void *x, double b_re, double b_im, void *y,
                  double *norm2_out);
+// One Lanczos update with the scalars on the device (dots: those of the
+// launch_apply that formed y): y = (y - alpha x) sc and
+// rec = {alpha, |y|^2, c, bpred}, where c is the z coefficient of the next
+// step's launch_apply.  k2 null: unit vectors, sc = bpred = 1, c = -|y|.
+// Otherwise x = sqrt(*k2) v: alpha from dots / *k2, bpred the next beta as
+// the dots predict it, sc = 1 / (sqrt(*k2) bpred).
+int launch_lanczos_update(el_ctx *ctx, int dtype, int64_t len, const void *x, void *y, const double *dots,
+                          const double *k2, double *rec);
 // dots_out[j] = <V_j, w> for j < k (V: k vectors of length len, contiguous,
 // leading dimension ld); complex results as (re, im) pairs.
 int launch_gemv_t(el_ctx *ctx, int dtype, int64_t len, int k, const void *V,

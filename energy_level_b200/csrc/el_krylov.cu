@@ -33,11 +33,10 @@ int sync_read(el_ctx *ctx, const double *dev, int count, double *host) {
   return EL_OK;
 }
 
-struct LanczosOut {
-  std::vector<double> alpha, beta;  // beta[j] couples v_j and v_{j+1}
-  int steps = 0;
-  bool invariant = false;
-};
+// Lanczos steps queued before the host reads their scalars: several while a
+// step's kernels are shorter than the host's wait for them, one on long
+// vectors, where a step that turns out not to be needed costs more.
+int steps_ahead(size_t vector_bytes) { return vector_bytes <= ((size_t)16 << 20) ? 4 : 1; }
 
 }  // namespace
 
@@ -55,7 +54,8 @@ extern "C" int el_bounds(el_ctx *ctx, el_ham *h, int max_iter, double tol,
   char *buf = (char *)el::workspace(ctx, 0, 3 * vb);
   if (!buf) return EL_ENOMEM;
   void *vp = buf, *v = buf + vb, *w = buf + 2 * vb;
-  double *d_sc = ctx->d_scalars;  // [0..3] dots, [8] norm2
+  double *d_sc = ctx->d_scalars;  // [0..3] dots, [8] norm2, [9] = 1
+  double *d_one = d_sc + 9;
   int rc;
   if (dim == 1) {
     double d;
@@ -72,6 +72,8 @@ extern "C" int el_bounds(el_ctx *ctx, el_ham *h, int max_iter, double tol,
   if (rc) return rc;
   rc = el::launch_scale(ctx, dtype, dim, d_sc + 8, 1, v);
   if (rc) return rc;
+  ctx->h_scalars[0] = 1.0;
+  EL_CUDA_TRY(ctx, el::copy(ctx, d_one, ctx->h_scalars, sizeof(double), cudaMemcpyHostToDevice));
   EL_CUDA_TRY(ctx, cudaMemsetAsync(vp, 0, vb, ctx->stream));
   // large full bases: the tiled two-pass product (el_kpm_tma.cu) instead of
   // the row kernel, whose high-bit partners come from DRAM again and again
@@ -88,67 +90,66 @@ extern "C" int el_bounds(el_ctx *ctx, el_ham *h, int max_iter, double tol,
   // The stored vectors are s_j = kappa_j v_j (v_j the unit Lanczos vectors):
   // one fused update per step forms s_{j+1} = (y - alpha s_j) / (kappa_j
   // beta_pred) with beta_pred from the step's dots, and its norm gives the
-  // exact beta and kappa_{j+1}; no separate normalisation pass.
+  // exact beta and kappa_{j+1}; no separate normalisation pass.  Every
+  // scalar of a step stays on the device (rec: alpha, kappa_{j+1}^2, the next
+  // step's z coefficient, beta_pred), so short vectors' steps are queued a
+  // few at a time and the host reads their scalars together: on 121,393 rows
+  // (57 steps) the two waits per step cost more than the step's kernels.
+  const int maxit = (int)std::min<int64_t>(max_iter, dim);
+  double *rec = (double *)el::workspace(ctx, 16, (size_t)(maxit + 1) * 4 * sizeof(double));
+  if (!rec) return EL_ENOMEM;
+  const int ahead = plan ? 1 : steps_ahead(vb);
   double kappa = 1.0, kappa_prev = 1.0;
   int stable = 0;
-  const int maxit = (int)std::min<int64_t>(max_iter, dim);
-  for (int j = 0; j < maxit; ++j) {
+  bool done = false;
+  std::vector<double> hr;
+  for (int j = 0; j < maxit && !done;) {
     if (el::cancelled(ctx)) return fail(ctx, EL_ECANCEL, "cancelled");
-    // y = H s_j - beta_j (kappa_j / kappa_{j-1}) s_{j-1} = kappa_j w_j
-    const double cz = j ? -beta * kappa / kappa_prev : 0.0;
-    if (plan) {
-      rc = el::hv_tiled(ctx, h, plan, iv, iw, ivp, cz, d_sc);
-    } else {
-      ApplyArgs A;
-      memset(&A, 0, sizeof A);
-      A.dtype = dtype; A.nvec = 1; A.x = v; A.z = vp; A.y = w;
-      A.a = 1.0; A.b = 0.0; A.c = cz; A.dots = d_sc; A.want_dots = 7;
-      rc = el::launch_apply(ctx, h, A);
-    }
-    if (rc) return rc;
-    double dots[4];
-    rc = sync_read(ctx, d_sc, 4, dots);
-    if (rc) return rc;
-    const double k2 = kappa * kappa;
-    const double alpha = dots[1] / k2;
-    const double bp2 = dots[3] / k2 - alpha * alpha;   // |w_j - alpha v_j|^2 from <y,y> (dots[3])
-    const double scale_a = std::max(1.0, std::fabs(alpha));
-    const bool fused = bp2 > 1e-6 * scale_a * scale_a;  // else: form the norm directly
-    const double bpred = fused ? std::sqrt(bp2) : 1.0;
-    const double sc = 1.0 / (kappa * bpred);
-    rc = el::launch_axpby(ctx, dtype, dim, -alpha * sc, 0, v, sc, 0, w, d_sc + 8);
-    if (rc) return rc;
-    double n2;
-    rc = sync_read(ctx, d_sc + 8, 1, &n2);
-    if (rc) return rc;
-    al.push_back(alpha);
-    // |s_{j+1}|^2 = n2 and s_{j+1} = (beta / bpred) v_{j+1}
-    const double kappa_next = std::sqrt(std::max(n2, 0.0));
-    beta = kappa_next * bpred;
-    const int m = (int)al.size();
-    double lo = el::tridiag_eig(al.data(), be.data(), m, 0);
-    double hi = el::tridiag_eig_max(al.data(), be.data(), m);
-    const double scale = std::max(1.0, std::max(std::fabs(lo), std::fabs(hi)));
-    if (m > 2 && std::fabs(lo - lo_prev) <= tol * scale && std::fabs(hi - hi_prev) <= tol * scale) {
-      if (++stable >= 3) { lo_prev = lo; hi_prev = hi; break; }
-    } else {
-      stable = 0;
-    }
-    lo_prev = lo;
-    hi_prev = hi;
-    if (beta <= 1e-13 * scale) break;  // invariant subspace: exact extremes
-    be.push_back(beta);
-    // s_{j-1} <- s_j ; s_j <- s_{j+1}
-    std::swap(vp, v);
-    std::swap(v, w);
-    std::swap(ivp, iv);
-    std::swap(iv, iw);
-    kappa_prev = kappa;
-    kappa = kappa_next;
-    if (!fused) {   // bring the vector to unit length before the next step
-      rc = el::launch_axpby(ctx, dtype, dim, 0, 0, nullptr, 1.0 / kappa, 0, v, nullptr);
+    const int nb = std::min(ahead, maxit - j);
+    for (int q = j; q < j + nb; ++q) {
+      // y = H s_j - beta_j (kappa_j / kappa_{j-1}) s_{j-1} = kappa_j w_j
+      if (plan) {
+        rc = el::hv_tiled(ctx, h, plan, iv, iw, ivp, q ? -beta * kappa / kappa_prev : 0.0, d_sc);
+      } else {
+        ApplyArgs A;
+        memset(&A, 0, sizeof A);
+        A.dtype = dtype; A.nvec = 1; A.x = v; A.z = vp; A.y = w;
+        A.a = 1.0; A.b = 0.0; A.c_dev = q ? rec + 4 * (q - 1) + 2 : nullptr; A.dots = d_sc; A.want_dots = 7;
+        rc = el::launch_apply(ctx, h, A);
+      }
       if (rc) return rc;
-      kappa = 1.0;
+      rc = el::launch_lanczos_update(ctx, dtype, dim, v, w, d_sc, q ? rec + 4 * (q - 1) + 1 : d_one, rec + 4 * q);
+      if (rc) return rc;
+      // s_{j-1} <- s_j ; s_j <- s_{j+1}
+      std::swap(vp, v);
+      std::swap(v, w);
+      std::swap(ivp, iv);
+      std::swap(iv, iw);
+    }
+    hr.resize(4 * nb);
+    rc = sync_read(ctx, rec + 4 * j, 4 * nb, hr.data());
+    if (rc) return rc;
+    for (int q = 0; q < nb && !done; ++q, ++j) {
+      const double alpha = hr[4 * q], n2 = hr[4 * q + 1], bpred = hr[4 * q + 3];
+      al.push_back(alpha);
+      // |s_{j+1}|^2 = n2 and s_{j+1} = (beta / bpred) v_{j+1}
+      const double kappa_next = std::sqrt(std::max(n2, 0.0));
+      beta = kappa_next * bpred;
+      const int m = (int)al.size();
+      const double lo = el::tridiag_eig(al.data(), be.data(), m, 0);
+      const double hi = el::tridiag_eig_max(al.data(), be.data(), m);
+      const double scale = std::max(1.0, std::max(std::fabs(lo), std::fabs(hi)));
+      if (m > 2 && std::fabs(lo - lo_prev) <= tol * scale && std::fabs(hi - hi_prev) <= tol * scale) {
+        if (++stable >= 3) done = true;
+      } else {
+        stable = 0;
+      }
+      lo_prev = lo;
+      hi_prev = hi;
+      if (beta <= 1e-13 * scale) done = true;  // invariant subspace: exact extremes
+      be.push_back(beta);
+      kappa_prev = kappa;
+      kappa = kappa_next;
     }
   }
   if (plan) {
@@ -288,6 +289,9 @@ extern "C" int el_lanczos_ground(el_ctx *ctx, el_ham *h, int dtype, const void *
   double *d_sc = ctx->d_scalars;           // [0..3] dots, [8] norm2
   double *d_coef = ctx->d_scalars + 64;    // [2*(m+1)] reorth coefficients
   if (2 * (m + 1) + 64 > EL_SCALARS) return fail(ctx, EL_EINVAL, "max_iter too large (<= %d)", EL_SCALARS / 2 - 40);
+  double *rec = (double *)el::workspace(ctx, 16, (size_t)(m + 1) * 4 * sizeof(double));
+  if (!rec) return EL_ENOMEM;
+  std::vector<double> hr;
   auto Vj = [&](int j) { return (void *)(Vb + (size_t)j * vb); };
   int rc;
   // start vector
@@ -319,30 +323,44 @@ extern "C" int el_lanczos_ground(el_ctx *ctx, el_ham *h, int dtype, const void *
     int j = 0;
     bool invariant = false;
     int last_check = -1;
+    // Steps [j, queued) are on the stream: H v_j - beta v_{j-1} with its dot,
+    // the update and the scaling of v_{j+1}, all scalars on the device
+    // (rec: alpha, |w|^2, -beta, -).  The host reads them together and goes
+    // through the steps in order; where one has to be reorthogonalised, the
+    // steps after it are queued again.
+    int queued = 0, read = 0;
     for (j = 0; j < m; ++j) {
       if (el::cancelled(ctx)) return fail(ctx, EL_ECANCEL, "cancelled");
       const double bj = j ? be[j - 1] : 0.0;
-      ApplyArgs A;
-      memset(&A, 0, sizeof A);
-      A.dtype = dtype; A.nvec = 1; A.x = Vj(j); A.z = j ? Vj(j - 1) : nullptr; A.y = w;
-      A.a = 1.0; A.c = -bj; A.dots = d_sc; A.want_dots = 2;
-      rc = el::launch_apply(ctx, h, A);
-      if (rc) return rc;
-      double dots[4];
-      rc = sync_read(ctx, d_sc, 4, dots);
-      if (rc) return rc;
-      const double alpha = dots[1];
+      if (j == queued) {
+        const int nb = std::min(force_next || reorth == 2 ? 1 : steps_ahead(vb), m - j);
+        for (int q = j; q < j + nb; ++q) {
+          ApplyArgs A;
+          memset(&A, 0, sizeof A);
+          A.dtype = dtype; A.nvec = 1; A.x = Vj(q); A.z = q ? Vj(q - 1) : nullptr; A.y = Vj(q + 1);
+          A.a = 1.0; A.c = -bj; A.c_dev = q > j ? rec + 4 * (q - 1) + 2 : nullptr; A.dots = d_sc; A.want_dots = 2;
+          rc = el::launch_apply(ctx, h, A);
+          if (rc) return rc;
+          rc = el::launch_lanczos_update(ctx, dtype, dim, Vj(q), Vj(q + 1), d_sc, nullptr, rec + 4 * q);
+          if (rc) return rc;
+          rc = el::launch_scale(ctx, dtype, dim, rec + 4 * q + 1, 1, Vj(q + 1));
+          if (rc) return rc;
+        }
+        hr.resize(4 * (size_t)nb);
+        rc = sync_read(ctx, rec + 4 * j, 4 * nb, hr.data());
+        if (rc) return rc;
+        queued = j + nb;
+        read = j;
+      }
+      const double alpha = hr[4 * (j - read)];
+      n2 = hr[4 * (j - read) + 1];
       al.push_back(alpha);
-      rc = el::launch_axpby(ctx, dtype, dim, -alpha, 0, Vj(j), 1, 0, w, d_sc + 8);
-      if (rc) return rc;
       // reorthogonalisation decision
       const bool forced = force_next;
       bool do_reorth = (reorth == 2) || forced;
       double anorm = 0.0;
       for (size_t q = 0; q < al.size(); ++q) anorm = std::max(anorm, std::fabs(al[q]));
       for (size_t q = 0; q < be.size(); ++q) anorm = std::max(anorm, std::fabs(be[q]));
-      rc = sync_read(ctx, d_sc + 8, 1, &n2);
-      if (rc) return rc;
       double bnext = std::sqrt(std::max(n2, 0.0));
       if (reorth == 1 && j > 0 && bnext > 0) {
         // omega(j+1, k) per Simon (1984), k = 0..j-1
@@ -363,18 +381,22 @@ extern "C" int el_lanczos_ground(el_ctx *ctx, el_ham *h, int dtype, const void *
         if (wmax > std::sqrt(eps)) do_reorth = true;
       }
       force_next = false;
-      if (do_reorth && j > 0) {
+      if (do_reorth && j > 0 && bnext > 0) {
+        // v_{j+1} = w / bnext is orthogonalised in place and scaled again
         for (int pass = 0; pass < 2; ++pass) {
-          rc = el::launch_gemv_t(ctx, dtype, dim, j + 1, Vb, dim, w, d_coef);
+          rc = el::launch_gemv_t(ctx, dtype, dim, j + 1, Vb, dim, Vj(j + 1), d_coef);
           if (rc) return rc;
-          rc = el::launch_gemv_n_sub(ctx, dtype, dim, j + 1, Vb, dim, d_coef, w);
+          rc = el::launch_gemv_n_sub(ctx, dtype, dim, j + 1, Vb, dim, d_coef, Vj(j + 1));
           if (rc) return rc;
         }
-        rc = el::launch_axpby(ctx, dtype, dim, 0, 0, nullptr, 1, 0, w, d_sc + 8);
+        rc = el::launch_axpby(ctx, dtype, dim, 0, 0, nullptr, 1, 0, Vj(j + 1), d_sc + 8);
+        if (rc) return rc;
+        rc = el::launch_scale(ctx, dtype, dim, d_sc + 8, 1, Vj(j + 1));
         if (rc) return rc;
         rc = sync_read(ctx, d_sc + 8, 1, &n2);
         if (rc) return rc;
-        bnext = std::sqrt(std::max(n2, 0.0));
+        bnext *= std::sqrt(std::max(n2, 0.0));
+        queued = j + 1;         // the steps after this one started from the old vector
         if (reorth == 1) {
           for (int k = 0; k <= j; ++k) wnext[k] = eps;
           wnext[j + 1] = 1.0;
@@ -404,9 +426,6 @@ extern "C" int el_lanczos_ground(el_ctx *ctx, el_ham *h, int dtype, const void *
         if (ok || invariant || last) { j = mm; break; }
       }
       be.push_back(bnext);
-      // v_{j+1} = w / beta
-      rc = el::launch_axpby(ctx, dtype, dim, 1.0 / bnext, 0, w, 0, 0, Vj(j + 1), nullptr);
-      if (rc) return rc;
     }
     const int mm = (int)al.size();
     // Ritz vectors and true residuals

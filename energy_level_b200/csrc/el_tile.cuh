@@ -70,7 +70,7 @@ __device__ __forceinline__ void finish_chunk(const KArgs &K, int64_t e, const Ch
   for (int w = 0; w < CW; ++w) y.v[w] = a * h.v[w] + b * x.v[w];
   if (K.z) {
     const V z = load_cs<S, CW>(reinterpret_cast<const V *>(K.z) + e);
-    const S c = (S)K.c;
+    const S c = (S)coef_c(K);
 #pragma unroll
     for (int w = 0; w < CW; ++w) y.v[w] += c * z.v[w];
   }
