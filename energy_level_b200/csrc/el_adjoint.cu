@@ -221,7 +221,7 @@ __global__ void k_step_bounds(BasisDev B, const double *__restrict__ diagV, Step
     for (int q = 0; q < B.n; ++q)
       if (el::flip_target(B, code1, r1, q) >= 0) flips1 |= 1ULL << q;
   }
-  for (int k = 0; k < K; ++k) {
+  for (int k = blockIdx.y; k < K; k += gridDim.y) {
     const double o = om[k], d0 = dl[k];
     double lo = 1e300, hi = -1e300;
     for (int64_t r = r1; r < B.dim; r += (int64_t)gridDim.x * blockDim.x) {
@@ -273,7 +273,10 @@ int step_bounds(el_ctx *ctx, el_ham *h, int K, const double *omega_k, const doub
   StepShapes sh;
   memset(&sh, 0, sizeof sh);
   for (int q = 0; q < n; ++q) { sh.a[q] = ash[n - 1 - q]; sh.b[q] = bsh[n - 1 - q]; }
-  k_step_bounds<<<grid, 256, 0, ctx->stream>>>(el::basis_dev(h->basis), h->d_diagV64, sh, K, d_om, d_dl, d_out);
+  // one row per thread leaves most of the GPU idle on small bases: the steps
+  // spread over grid columns (60 x 200 steps in turn 545 us, 16 columns 60 us)
+  const int cols = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(K, 16), 8 * (int64_t)sms / grid));
+  k_step_bounds<<<dim3(grid, cols), 256, 0, ctx->stream>>>(el::basis_dev(h->basis), h->d_diagV64, sh, K, d_om, d_dl, d_out);
   ctx->launches++;
   EL_LAUNCH_CHECK(ctx);
   std::vector<double> part((size_t)grid * K * 2);
@@ -288,6 +291,8 @@ int step_bounds(el_ctx *ctx, el_ham *h, int K, const double *omega_k, const doub
     }
   return EL_OK;
 }
+
+constexpr size_t STORE_MAX = (size_t)1 << 30;   // bytes of Chebyshev terms kept between the two passes
 
 template <typename S>
 int adjoint_impl(el_ctx *ctx, el_ham *h, int dtype, int K, const double *tau, const double *omega_k,
@@ -320,8 +325,16 @@ int adjoint_impl(el_ctx *ctx, el_ham *h, int dtype, int K, const double *tau, co
       Mmax = std::max(Mmax, plans[k].M);
     }
   }
-  // workspace: K+1 checkpoints, Mmax+1 terms, 3 adjoint vectors, lambda
-  char *buf = (char *)el::workspace(ctx, 11, (size_t)(K + 1 + Mmax + 1 + 4) * vb);
+  // workspace: K+1 checkpoints, Mmax+1 terms (of every step in the cooperative
+  // gradient, while they fit STORE_MAX), 3 adjoint vectors, lambda
+  const bool coop = ctx->adjoint_mode != EL_ADJ_STREAM;
+  bool stored = coop && (size_t)K * (Mmax + 1) * vb <= STORE_MAX;
+  char *buf = nullptr;
+  if (stored) {
+    buf = (char *)el::workspace(ctx, 11, (size_t)(K + 1 + (size_t)K * (Mmax + 1) + 4) * vb);
+    if (!buf) stored = false;      // no room: form the terms again in the reverse pass
+  }
+  if (!buf) buf = (char *)el::workspace(ctx, 11, (size_t)(K + 1 + Mmax + 1 + 4) * vb);
   if (!buf) return EL_ENOMEM;
   auto ckp = [&](int k) { return (void *)(buf + (size_t)k * vb); };
   char *tb = buf + (size_t)(K + 1) * vb;
@@ -329,12 +342,12 @@ int adjoint_impl(el_ctx *ctx, el_ham *h, int dtype, int K, const double *tau, co
   char *ub = tb + (size_t)(Mmax + 1) * vb;
   void *U[3] = {ub, ub + vb, ub + 2 * vb};
   void *lam = ub + 3 * vb;
-  if (ctx->adjoint_mode != EL_ADJ_STREAM) {
+  if (coop) {
     // one cooperative launch for the whole gradient
     std::vector<double> hg;
     double F = 0.0;
     int rc = el::adjoint_coop<S>(ctx, h, K, plans, Mmax, omega_k, delta_k, ash, bsh, psi0, target, obs_diag,
-                                 buf, hg, F);
+                                 buf, stored, hg, F);
     if (rc) return rc;
     if (psi_final) {
       EL_CUDA_TRY(ctx, el::copy(ctx, psi_final, ckp(K), vb, cudaMemcpyDeviceToDevice));
@@ -343,15 +356,8 @@ int adjoint_impl(el_ctx *ctx, el_ham *h, int dtype, int K, const double *tau, co
     rc = set_drive(0);   // the drive the stream path leaves behind
     if (rc) return rc;
     for (int k = 0; k < K; ++k) {
-      const el::ChebPlan &pl = plans[k];
-      double go = 0.0, gd = 0.0;
-      for (int m = 1; m <= pl.M; ++m) {
-        const double s = (m == 1) ? 1.0 : 2.0;
-        go += s * hg[((size_t)k * (Mmax + 1) + m) * 2];
-        gd += s * hg[((size_t)k * (Mmax + 1) + m) * 2 + 1];
-      }
-      gO_out[k] = 2.0 * go / pl.a;
-      gD_out[k] = 2.0 * gd / pl.a;
+      gO_out[k] = 2.0 * hg[2 * (size_t)k] / plans[k].a;
+      gD_out[k] = 2.0 * hg[2 * (size_t)k + 1] / plans[k].a;
     }
     *F_out = F;
     return EL_OK;

@@ -1,8 +1,7 @@
 // The whole adjoint pulse gradient in one cooperative launch.
 //
-// Same mathematics as el_adjoint.cu (forward Chebyshev steps with one
-// checkpoint per step, the objective and lambda_K, then per step the terms
-// t_0..t_{M-1} recomputed from the checkpoint and the reverse recurrence
+// Same mathematics as el_adjoint.cu (forward Chebyshev steps, the objective
+// and lambda_K, then per step the reverse recurrence
 //     u_M = conj(c_M) lambda,
 //     u_m = conj(c_m) lambda + (s/a) (H - b) u_{m+1} - u_{m+2}
 // with the gradient dots Re<G_Omega u_{m+1}, t_m>, Re<G_Delta u_{m+1}, t_m>),
@@ -10,13 +9,20 @@
 // kernel, separated by grid barriers, instead of one launch: the bases the
 // pulse gradient runs on hold tens of thousands of rows, so the separate
 // launches of the stream path (about 3 K M of them) cost more than their
-// work.  Four lanes share a row (its flips split between them) as in
-// k_adjoint_step, and keep its flip targets in registers across all
-// sweeps; every step's Chebyshev plan (a, b, M, c_m) is computed on
-// the host first and read from device arrays.  Gradient dots go to per-CTA
-// slots [step][m][CTA] that the host adds up in a fixed order, so the
-// result does not depend on scheduling.  Grid-barrier waits are bounded: a
-// wait that runs out sets an error flag, every later barrier returns at
+// work.  A phase is a barrier and a chain of L2 reads whatever it computes
+// (2.0 us on 15,127 rows), so their number counts: the forward pass keeps
+// every term t_m of every step while all of them fit STORE_MAX bytes (318 MB
+// for 200 steps on that basis; otherwise the reverse pass forms them again
+// from the step's checkpoint, another 1827 of 7186 phases), a step's last
+// reverse phase also writes lambda and the next step's u_M, and each thread
+// adds up its gradient dots over a step, one block sum per step.  20-site
+// ring, 200 steps, complex64: 22.5 -> 11.2 ms (14.9 with the row values read from memory in each phase).  Four lanes share a row (its
+// flips split between them) as in k_adjoint_step, and keep its flip targets
+// in registers across all sweeps; every step's Chebyshev plan (a, b, M, c_m)
+// is computed on the host first and read from device arrays.  Gradient dots
+// go to per-CTA slots [step][CTA] that the host adds up in a fixed order, so
+// the result does not depend on scheduling.  Grid-barrier waits are bounded:
+// a wait that runs out sets an error flag, every later barrier returns at
 // once, and the host reports EL_ECUDA.
 #include "el_internal.cuh"
 
@@ -41,12 +47,13 @@ struct CoopAdj {
   S ahalf[EL_MAX_SITES];   // a_i / 2 per bit position
   S bsh[EL_MAX_SITES];     // b_i per bit position
   S *ckp;                  // [K + 1][dim] complex checkpoints
-  S *term;                 // [Mmax + 1][dim] complex Chebyshev terms
+  S *term;                 // [Mmax + 1][dim] complex Chebyshev terms, of every step if stored
+  int stored;
   S *U;                    // [3][dim] complex adjoint vectors
   S *lam;                  // [dim] complex
   const S *target;         // fidelity target, or null
   const double *obs;       // diagonal observable, or null
-  double *part;            // [K][Mmax + 1][nctas][2] gradient dots per CTA
+  double *part;            // [K][nctas][2] gradient dots per CTA, summed over a step's terms
   double *fpart;           // [nctas][2] objective partials
   double *fout;            // [2]: <target, psi_K> (or F, 0)
   unsigned *bar;           // arrival counter, zero at launch
@@ -162,7 +169,8 @@ struct Sweep {
   const S *x, *z, *lam, *t;
   S *y, *acc;
   S alpha, beta, clr, cli, wr, wi, w0r, w0i;
-  int acc_mode;
+  int acc_mode;          // 3: acc = y, and y is stored times (wr, wi)
+  double gw;             // weight of the gradient dots
 };
 
 template <typename S>
@@ -209,8 +217,15 @@ __device__ __forceinline__ void sweep(const CoopAdj<S> &P, S om, S dl, const Swe
       yre += W.clr * lr - W.cli * li;
       yim += W.clr * li + W.cli * lr;
     }
-    W.y[2 * r] = yre;
-    W.y[2 * r + 1] = yim;
+    if (W.acc_mode == 3) {
+      W.acc[2 * r] = yre;
+      W.acc[2 * r + 1] = yim;
+      W.y[2 * r] = W.wr * yre - W.wi * yim;
+      W.y[2 * r + 1] = W.wr * yim + W.wi * yre;
+    } else {
+      W.y[2 * r] = yre;
+      W.y[2 * r + 1] = yim;
+    }
     if (W.acc_mode == 1) {
       W.acc[2 * r] = W.w0r * xr - W.w0i * xi + W.wr * yre - W.wi * yim;
       W.acc[2 * r + 1] = W.w0r * xi + W.w0i * xr + W.wr * yim + W.wi * yre;
@@ -220,8 +235,174 @@ __device__ __forceinline__ void sweep(const CoopAdj<S> &P, S om, S dl, const Swe
     }
     if (W.t) {
       const double tr = W.t[2 * r], ti = W.t[2 * r + 1];
-      gO += (double)sre * tr + (double)sim * ti;                  // Re(conj(G_O x) t)
-      gD += -(double)nb * ((double)xr * tr + (double)xi * ti);    // Re(conj(G_D x) t)
+      gO += W.gw * ((double)sre * tr + (double)sim * ti);               // Re(conj(G_O x) t)
+      gD -= W.gw * (double)nb * ((double)xr * tr + (double)xi * ti);    // Re(conj(G_D x) t)
+    }
+  }
+}
+
+// The whole gradient where one pass of the grid covers the basis and every
+// term is stored: a row's own values (t_m and t_{m-1}, the accumulated state,
+// u_{m+1}, u_{m+2}, lambda, its diagonal) stay in registers of the row's first
+// lane, a step's coefficients come through shared memory, and the stored
+// term of the next phase is read before the barrier.  What a phase waits for
+// after its barrier is one round of flip partners.
+constexpr int MAXC = 256;   // terms of a step held in shared memory
+
+template <typename S>
+__device__ __forceinline__ void gather_flips(const RowCache<S> &rc, const S *x, S &re, S &im) {
+  typedef typename VecT<S, true>::type V2;
+  V2 v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (rc.tg[q] >= 0) v[q] = reinterpret_cast<const V2 *>(x)[rc.tg[q]];
+  re = S(0);
+  im = S(0);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    if (rc.tg[q] < 0) continue;
+    re += rc.amp[q] * v[q].x;
+    im += rc.amp[q] * v[q].y;
+  }
+#pragma unroll
+  for (int off = CL / 2; off > 0; off >>= 1) {
+    re += __shfl_xor_sync(0xffffffffu, re, off);
+    im += __shfl_xor_sync(0xffffffffu, im, off);
+  }
+}
+
+template <typename S>
+__device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, double *red, unsigned &gen) {
+  typedef typename VecT<S, true>::type V2;
+  __shared__ S cbuf[2][2 * MAXC];
+  __shared__ double s_ov[2];
+  const size_t vs = (size_t)P.B.dim * 2;
+  const bool mine = rc.active && (threadIdx.x & (CL - 1)) == 0;   // this thread finishes the row
+  const int64_t r = rc.r;
+  auto sync = [&]() { coop_sync(P.bar, P.err, P.nctas, P.poll_limit, gen); };
+  auto at = [&](const S *p) { return reinterpret_cast<const V2 *>(p)[r]; };
+  auto put = [&](S *p, S re, S im) { V2 v; v.x = re; v.y = im; reinterpret_cast<V2 *>(p)[r] = v; };
+  // coefficients of step k into buffer k & 1 (read after the next barrier)
+  auto fetch = [&](int k) {
+    if (k < 0 || k >= P.K) return;
+    const double *c = P.pc + (size_t)k * (P.Mmax + 1) * 2;
+    for (int q = threadIdx.x; q < 2 * (P.pm[k] + 1); q += CNT) cbuf[k & 1][q] = (S)c[q];
+  };
+  const S diag = P.diagV[r];
+  V2 x0 = at(P.ckp);
+  S xr = x0.x, xi = x0.y;       // own value of the vector the next sweep gathers
+  fetch(0);
+  __syncthreads();
+  // ---- forward
+  for (int k = 0; k < P.K; ++k) {
+    const S a = (S)P.pa[k], b = (S)P.pb[k], om = (S)P.om[k];
+    const S d = diag + (S)P.dl[k] * rc.nb;
+    const int M = P.pm[k];
+    const S *c = cbuf[k & 1];
+    S *term = P.term + (size_t)k * (P.Mmax + 1) * vs;
+    S *out = P.ckp + (size_t)(k + 1) * vs;
+    const S *x = P.ckp + (size_t)k * vs;
+    S zr = S(0), zi = S(0);
+    S accr = c[0] * xr - c[1] * xi, acci = c[0] * xi + c[1] * xr;
+    for (int m = 1; m <= M; ++m) {
+      S re, im;
+      gather_flips<S>(rc, x, re, im);
+      const S al = (m == 1 ? S(1) : S(2)) / a, be = (m == 1 ? -b : S(-2) * b) / a;
+      const S yr = al * (d * xr + om * re) + be * xr - zr, yi = al * (d * xi + om * im) + be * xi - zi;
+      accr += c[2 * m] * yr - c[2 * m + 1] * yi;
+      acci += c[2 * m] * yi + c[2 * m + 1] * yr;
+      zr = xr; zi = xi;
+      xr = yr; xi = yi;
+      x = term + (size_t)m * vs;
+      if (m < M) {
+        if (mine) put(term + (size_t)m * vs, yr, yi);
+      } else {
+        if (mine) put(out, accr, acci);
+        xr = accr;
+        xi = acci;
+      }
+      if (m == 1) fetch(k + 1);
+      sync();
+    }
+  }
+  // ---- objective, lambda_K and u_M of the last step
+  S lr = S(0), li = S(0);
+  {
+    double fa = 0.0, fb = 0.0;
+    if (mine) {
+      if (P.target) {
+        const V2 t = at(P.target);
+        fa = (double)t.x * xr + (double)t.y * xi;   // conj(target) psi
+        fb = (double)t.x * xi - (double)t.y * xr;
+      } else {
+        fa = P.obs[r] * ((double)xr * xr + (double)xi * xi);
+      }
+    }
+    block_sum2(fa, fb, red, P.fpart + 2 * blockIdx.x);
+    sync();
+    double sa = 0.0, sb = 0.0;
+    for (int i = threadIdx.x; i < P.nctas; i += CNT) { sa += __ldcg(&P.fpart[2 * i]); sb += __ldcg(&P.fpart[2 * i + 1]); }
+    block_sum2(sa, sb, red, s_ov);
+    if (blockIdx.x == 0 && threadIdx.x == 0) { P.fout[0] = s_ov[0]; P.fout[1] = s_ov[1]; }
+    if (P.target) {   // lambda = <target, psi> target
+      const V2 t = at(P.target);
+      lr = (S)s_ov[0] * t.x - (S)s_ov[1] * t.y;
+      li = (S)s_ov[0] * t.y + (S)s_ov[1] * t.x;
+    } else {          // lambda = O psi
+      lr = (S)P.obs[r] * xr;
+      li = (S)P.obs[r] * xi;
+    }
+    const S *c = cbuf[(P.K - 1) & 1];
+    const int M = P.pm[P.K - 1];
+    xr = c[2 * M] * lr + c[2 * M + 1] * li;       // conj(c_M) lambda
+    xi = c[2 * M] * li - c[2 * M + 1] * lr;
+    if (mine) put(P.U, xr, xi);
+    fetch(P.K - 2);
+    sync();
+  }
+  // ---- backward
+  int us = 0;
+  for (int k = P.K - 1; k >= 0; --k) {
+    const S a = (S)P.pa[k], b = (S)P.pb[k], om = (S)P.om[k];
+    const S d = diag + (S)P.dl[k] * rc.nb;
+    const int M = P.pm[k], Mn = k > 0 ? P.pm[k - 1] : 0;
+    const S *c = cbuf[k & 1], *cn = cbuf[(k & 1) ^ 1];
+    const S *term = P.term + (size_t)k * (P.Mmax + 1) * vs;
+    S zr = S(0), zi = S(0);
+    double gO = 0.0, gD = 0.0;
+    if (M == 1 && k + 1 < P.K) {   // one phase: the next step's coefficients are needed in it
+      fetch(k - 1);
+      __syncthreads();
+    }
+    V2 t = at(M - 1 == 0 ? P.ckp + (size_t)k * vs : term + (size_t)(M - 1) * vs);
+    for (int m = M - 1; m >= 0; --m) {
+      S re, im;
+      gather_flips<S>(rc, P.U + (size_t)us * vs, re, im);
+      const S al = (m == 0 ? S(1) : S(2)) / a, be = (m == 0 ? -b : S(-2) * b) / a;
+      // conj(c_m) lambda + (s/a)(H - b) u_{m+1} - u_{m+2}
+      const S yr = al * (d * xr + om * re) + be * xr - zr + (c[2 * m] * lr + c[2 * m + 1] * li);
+      const S yi = al * (d * xi + om * im) + be * xi - zi + (c[2 * m] * li - c[2 * m + 1] * lr);
+      if (mine) {
+        const double w = (m == 0) ? 1.0 : 2.0, tr = t.x, ti = t.y;
+        gO += w * ((double)re * tr + (double)im * ti);                       // Re(conj(G_O u) t)
+        gD -= w * (double)rc.nb * ((double)xr * tr + (double)xi * ti);       // Re(conj(G_D u) t)
+      }
+      us = us == 2 ? 0 : us + 1;
+      zr = xr; zi = xi;
+      if (m > 0) {
+        xr = yr;
+        xi = yi;
+        t = at(m == 1 ? P.ckp + (size_t)k * vs : term + (size_t)(m - 1) * vs);   // for the next phase
+      } else {   // lambda_{k-1} = u_0, published as u_M of step k - 1
+        lr = yr;
+        li = yi;
+        xr = cn[2 * Mn] * lr + cn[2 * Mn + 1] * li;
+        xi = cn[2 * Mn] * li - cn[2 * Mn + 1] * lr;
+        block_sum2(gO, gD, red, P.part + ((size_t)k * P.nctas + blockIdx.x) * 2);
+      }
+      if (mine) put(P.U + (size_t)us * vs, xr, xi);
+      if (M > 1 && m == M - 1 && k + 1 < P.K) fetch(k - 1);   // step k + 1's buffer is done with
+      sync();
     }
   }
 }
@@ -242,6 +423,10 @@ __global__ void __launch_bounds__(CNT, 2) k_adjoint_coop(const CoopAdj<S> P) {
   RowCache<S> cache;
   const bool one_pass = dim <= (int64_t)gridDim.x * (CNT / CL) && P.B.n <= 8 * CL;
   if (one_pass) row_cache<S>(P, cache);
+  if (one_pass && P.stored && P.Mmax < MAXC) {
+    gradient_one_pass<S>(P, cache, red, gen);
+    return;
+  }
   // ---- forward: psi_{k+1} = sum_m c_m T_m(Htil_k) psi_k
   for (int k = 0; k < P.K; ++k) {
     const S a = (S)P.pa[k], b = (S)P.pb[k];
@@ -250,17 +435,18 @@ __global__ void __launch_bounds__(CNT, 2) k_adjoint_coop(const CoopAdj<S> P) {
     const S om = (S)P.om[k], dl = (S)P.dl[k];
     const S *x0 = P.ckp + (size_t)k * vs;
     S *out = P.ckp + (size_t)(k + 1) * vs;
+    S *term = P.term + (P.stored ? (size_t)k * (P.Mmax + 1) * vs : 0);
     Sweep<S> W{};
-    W.x = x0; W.y = P.term + vs; W.acc = out; W.acc_mode = 1;
+    W.x = x0; W.y = term + vs; W.acc = out; W.acc_mode = 1;
     W.alpha = S(1) / a; W.beta = -b / a;
     W.w0r = (S)c[0]; W.w0i = (S)c[1]; W.wr = (S)c[2]; W.wi = (S)c[3];
     sweep<S>(P, om, dl, W, g0, g1, cache, one_pass);
     sync();
     for (int m = 2; m <= M; ++m) {
       Sweep<S> V{};
-      V.x = P.term + (size_t)(m - 1) * vs;
-      V.z = (m == 2) ? x0 : P.term + (size_t)(m - 2) * vs;
-      V.y = P.term + (size_t)m * vs;
+      V.x = term + (size_t)(m - 1) * vs;
+      V.z = (m == 2) ? x0 : term + (size_t)(m - 2) * vs;
+      V.y = term + (size_t)m * vs;
       V.acc = out; V.acc_mode = 2;
       V.alpha = S(2) / a; V.beta = S(-2) * b / a;
       V.wr = (S)c[2 * m]; V.wi = (S)c[2 * m + 1];
@@ -293,86 +479,90 @@ __global__ void __launch_bounds__(CNT, 2) k_adjoint_coop(const CoopAdj<S> P) {
     }
     __syncthreads();
     const S ovr = (S)s_ov[0], ovi = (S)s_ov[1];
+    const double *cK = P.pc + ((size_t)(P.K - 1) * (P.Mmax + 1) + P.pm[P.K - 1]) * 2;
+    const S cr = (S)cK[0], ci = (S)(-cK[1]);
     for (int64_t r = (int64_t)blockIdx.x * CNT + threadIdx.x; r < dim; r += (int64_t)gridDim.x * CNT) {
+      S lr, li;
       if (P.target) {   // lambda = <target, psi> target
         const S tr = P.target[2 * r], ti = P.target[2 * r + 1];
-        P.lam[2 * r] = ovr * tr - ovi * ti;
-        P.lam[2 * r + 1] = ovr * ti + ovi * tr;
+        lr = ovr * tr - ovi * ti;
+        li = ovr * ti + ovi * tr;
       } else {          // lambda = O psi
         const S o = (S)P.obs[r];
-        P.lam[2 * r] = o * psi[2 * r];
-        P.lam[2 * r + 1] = o * psi[2 * r + 1];
+        lr = o * psi[2 * r];
+        li = o * psi[2 * r + 1];
       }
+      P.lam[2 * r] = lr;
+      P.lam[2 * r + 1] = li;
+      P.U[2 * r] = cr * lr - ci * li;       // u_M = conj(c_M) lambda of the last step
+      P.U[2 * r + 1] = cr * li + ci * lr;
     }
     sync();
   }
-  // ---- backward, one step at a time from the last
+  // ---- backward, one step at a time from the last; u_{m+1} is in slot us
+  int us = 0;
   for (int k = P.K - 1; k >= 0; --k) {
     const S a = (S)P.pa[k], b = (S)P.pb[k];
     const int M = P.pm[k];
     const double *c = P.pc + (size_t)k * (P.Mmax + 1) * 2;
     const S om = (S)P.om[k], dl = (S)P.dl[k];
     const S *x0 = P.ckp + (size_t)k * vs;
-    // t_1 .. t_{M-1} of this step again from its checkpoint (t_0 = x0)
-    for (int m = 1; m <= M - 1; ++m) {
-      Sweep<S> V{};
-      V.x = (m == 1) ? x0 : P.term + (size_t)(m - 1) * vs;
-      V.z = (m == 1) ? nullptr : ((m == 2) ? x0 : P.term + (size_t)(m - 2) * vs);
-      V.y = P.term + (size_t)m * vs;
-      V.alpha = (m == 1 ? S(1) : S(2)) / a;
-      V.beta = (m == 1 ? -b : S(-2) * b) / a;
-      sweep<S>(P, om, dl, V, g0, g1, cache, one_pass);
-      sync();
-    }
-    // u_M = conj(c_M) lambda
-    {
-      const S cr = (S)c[2 * M], ci = (S)(-c[2 * M + 1]);
-      S *uM = P.U + (size_t)(M % 3) * vs;
-      for (int64_t r = (int64_t)blockIdx.x * CNT + threadIdx.x; r < dim; r += (int64_t)gridDim.x * CNT) {
-        const S lr = P.lam[2 * r], li = P.lam[2 * r + 1];
-        uM[2 * r] = cr * lr - ci * li;
-        uM[2 * r + 1] = cr * li + ci * lr;
+    S *term = P.term + (P.stored ? (size_t)k * (P.Mmax + 1) * vs : 0);
+    if (!P.stored) {
+      // t_1 .. t_{M-1} of this step again from its checkpoint (t_0 = x0)
+      for (int m = 1; m <= M - 1; ++m) {
+        Sweep<S> V{};
+        V.x = (m == 1) ? x0 : term + (size_t)(m - 1) * vs;
+        V.z = (m == 1) ? nullptr : ((m == 2) ? x0 : term + (size_t)(m - 2) * vs);
+        V.y = term + (size_t)m * vs;
+        V.alpha = (m == 1 ? S(1) : S(2)) / a;
+        V.beta = (m == 1 ? -b : S(-2) * b) / a;
+        sweep<S>(P, om, dl, V, g0, g1, cache, one_pass);
+        sync();
       }
     }
-    sync();
     // u_m = conj(c_m) lambda + (s/a)(H - b) u_{m+1} - u_{m+2}, with the dots of u_{m+1} and t_m
+    double gO = 0.0, gD = 0.0;
     for (int m = M - 1; m >= 0; --m) {
       const S s = (m == 0) ? S(1) : S(2);
+      const int next = us == 2 ? 0 : us + 1, prev = us == 0 ? 2 : us - 1;
       Sweep<S> V{};
-      V.x = P.U + (size_t)((m + 1) % 3) * vs;
-      V.z = (m + 2 <= M) ? P.U + (size_t)((m + 2) % 3) * vs : nullptr;
-      V.y = P.U + (size_t)(m % 3) * vs;
+      V.x = P.U + (size_t)us * vs;
+      V.z = (m + 2 <= M) ? P.U + (size_t)prev * vs : nullptr;
+      V.y = P.U + (size_t)next * vs;
       V.lam = P.lam;
       V.clr = (S)c[2 * m];
       V.cli = (S)(-c[2 * m + 1]);
-      V.t = (m == 0) ? x0 : P.term + (size_t)m * vs;
+      V.t = (m == 0) ? x0 : term + (size_t)m * vs;
       V.alpha = s / a;
       V.beta = -s * b / a;
-      double gO = 0.0, gD = 0.0;
+      V.gw = (m == 0) ? 1.0 : 2.0;
+      if (m == 0) {   // lambda_{k-1} = u_0, and u_M of step k - 1 in the slot of u_0
+        const double *cn = P.pc + (k > 0 ? ((size_t)(k - 1) * (P.Mmax + 1) + P.pm[k - 1]) * 2 : 0);
+        V.acc = P.lam;
+        V.acc_mode = 3;
+        V.wr = (S)cn[0];
+        V.wi = (S)(-cn[1]);
+      }
       sweep<S>(P, om, dl, V, gO, gD, cache, one_pass);
-      block_sum2(gO, gD, red, P.part + (((size_t)k * (P.Mmax + 1) + (m + 1)) * P.nctas + blockIdx.x) * 2);
+      us = next;
+      if (m == 0) block_sum2(gO, gD, red, P.part + ((size_t)k * P.nctas + blockIdx.x) * 2);
       sync();
     }
-    // lambda_{k-1} = u_0
-    {
-      const S *u0 = P.U;
-      for (int64_t r = (int64_t)blockIdx.x * CNT + threadIdx.x; r < (int64_t)vs; r += (int64_t)gridDim.x * CNT)
-        P.lam[r] = u0[r];
-    }
-    sync();
   }
 }
 
 }  // namespace
 
 // Run the cooperative gradient; plans[k] are the steps' expansions.  Fills
-// hg[(k (Mmax + 1) + m) 2 + {0, 1}] (the per-term dots, as the stream path
-// does) and F.  EL_ECUDA when a grid-barrier wait ran out.
+// hg[2 k + {0, 1}] (the dots of step k summed over its terms with their
+// weights) and F.  stored: buf holds every step's terms.  EL_ECUDA when a
+// grid-barrier wait ran out.
 template <typename S>
 int adjoint_coop(el_ctx *ctx, el_ham *h, int K, const std::vector<ChebPlan> &plans, int Mmax,
                  const double *omega_k, const double *delta_k, const std::vector<double> &ash,
                  const std::vector<double> &bsh, const void *psi0, const void *target, const double *obs_diag,
-                 void *buf, std::vector<double> &hg, double &F) {
+                 void *buf, bool stored, std::vector<double> &hg, double &F) {
   const int n = h->n;
   const int64_t dim = h->basis->dim;
   const size_t vb = (size_t)dim * 2 * sizeof(S);
@@ -385,7 +575,7 @@ int adjoint_coop(el_ctx *ctx, el_ham *h, int K, const std::vector<ChebPlan> &pla
   const int nctas = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)per_sm * sms));
   // device tables: plans, drive, dots
   const size_t nplan = (size_t)K * (Mmax + 1) * 2;
-  const size_t nparts = (size_t)K * (Mmax + 1) * nctas * 2;
+  const size_t nparts = (size_t)K * nctas * 2;
   const size_t tab_doubles = 4 * (size_t)K + nplan + nparts + (size_t)nctas * 2 + 2;
   const size_t tab_bytes = tab_doubles * 8 + (size_t)K * 4 + 64;
   char *tb = (char *)el::workspace(ctx, 12, tab_bytes);
@@ -427,8 +617,10 @@ int adjoint_coop(el_ctx *ctx, el_ham *h, int K, const std::vector<ChebPlan> &pla
   }
   P.ckp = (S *)vbuf;
   P.term = (S *)(vbuf + (size_t)(K + 1) * vb);
-  P.U = (S *)(vbuf + (size_t)(K + 1 + Mmax + 1) * vb);
-  P.lam = (S *)(vbuf + (size_t)(K + 1 + Mmax + 1 + 3) * vb);
+  P.stored = stored ? 1 : 0;
+  const size_t nterms = (size_t)(stored ? K : 1) * (Mmax + 1);
+  P.U = (S *)(vbuf + (K + 1 + nterms) * vb);
+  P.lam = (S *)(vbuf + (K + 1 + nterms + 3) * vb);
   P.target = (const S *)target;
   P.obs = obs_diag;
   P.part = d_part; P.fpart = d_fpart; P.fout = d_fout;
@@ -445,25 +637,21 @@ int adjoint_coop(el_ctx *ctx, el_ham *h, int K, const std::vector<ChebPlan> &pla
   EL_CUDA_TRY(ctx, el::copy(ctx, hs, d_sync, 8, cudaMemcpyDeviceToHost));
   EL_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   if (hs[1]) return fail(ctx, EL_ECUDA, "cooperative adjoint: grid barrier timed out");
-  hg.assign((size_t)K * (Mmax + 1) * 2, 0.0);
+  hg.assign((size_t)K * 2, 0.0);
   for (int k = 0; k < K; ++k)
-    for (int m = 1; m <= plans[k].M; ++m)
-      for (int q = 0; q < 2; ++q) {
-        double s = 0.0;
-        for (int b = 0; b < nctas; ++b) s += parts[(((size_t)k * (Mmax + 1) + m) * nctas + b) * 2 + q];
-        hg[((size_t)k * (Mmax + 1) + m) * 2 + q] = s;
-      }
+    for (int b = 0; b < nctas; ++b)
+      for (int q = 0; q < 2; ++q) hg[2 * (size_t)k + q] += parts[((size_t)k * nctas + b) * 2 + q];
   F = target ? fo[0] * fo[0] + fo[1] * fo[1] : fo[0];
   return EL_OK;
 }
 
 template int adjoint_coop<float>(el_ctx *, el_ham *, int, const std::vector<ChebPlan> &, int, const double *,
                                  const double *, const std::vector<double> &, const std::vector<double> &,
-                                 const void *, const void *, const double *, void *, std::vector<double> &,
+                                 const void *, const void *, const double *, void *, bool, std::vector<double> &,
                                  double &);
 template int adjoint_coop<double>(el_ctx *, el_ham *, int, const std::vector<ChebPlan> &, int, const double *,
                                   const double *, const std::vector<double> &, const std::vector<double> &,
-                                  const void *, const void *, const double *, void *, std::vector<double> &,
+                                  const void *, const void *, const double *, void *, bool, std::vector<double> &,
                                   double &);
 
 }  // namespace el
