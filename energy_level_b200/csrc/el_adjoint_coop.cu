@@ -16,7 +16,7 @@
 // from the step's checkpoint, another 1827 of 7186 phases), a step's last
 // reverse phase also writes lambda and the next step's u_M, and each thread
 // adds up its gradient dots over a step, one block sum per step.  20-site
-// ring, 200 steps, complex64: 22.5 -> 11.2 ms (14.9 with the row values read from memory in each phase).  Four lanes share a row (its
+// ring, 200 steps, complex64: 22.8 -> 10.7 ms (14.9 with the row values read from memory in each phase).  Four lanes share a row (its
 // flips split between them) as in k_adjoint_step, and keep its flip targets
 // in registers across all sweeps; every step's Chebyshev plan (a, b, M, c_m)
 // is computed on the host first and read from device arrays.  Gradient dots
@@ -24,7 +24,7 @@
 // the result does not depend on scheduling.  Grid-barrier waits are bounded:
 // a wait that runs out sets an error flag, every later barrier returns at
 // once, and the host reports EL_ECUDA.
-#include "el_internal.cuh"
+#include "el_coop.cuh"
 
 #include <algorithm>
 
@@ -33,7 +33,7 @@ namespace el {
 namespace {
 
 constexpr int CL = 4;      // lanes per row
-constexpr int CNT = 256;   // threads per CTA
+constexpr int CNT = 512;   // threads per CTA: one CTA per SM; 256 (two) 5 % slower, twice the arrivals per barrier
 
 template <typename S>
 struct CoopAdj {
@@ -59,25 +59,6 @@ struct CoopAdj {
   unsigned *bar;           // arrival counter, zero at launch
   int *err;                // set when a barrier wait ran out
 };
-
-__device__ __forceinline__ void coop_sync(unsigned *bar, int *err, int nctas, int poll_limit, unsigned &gen) {
-  __syncthreads();
-  gen += (unsigned)nctas;
-  if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-    if (!*(volatile int *)err) {
-      int polls = 0;
-      unsigned v;
-      for (;;) {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-        if (v >= gen) break;
-        if (++polls > poll_limit) { atomicExch(err, 1); break; }
-        if ((polls & 255) == 0 && *(volatile int *)err) break;
-      }
-    }
-  }
-  __syncthreads();
-}
 
 // The flip sum (sum over allowed flips of a_i/2 x[target], complex) and
 // nb = sum of b_i over the set sites of a row, reduced over the CL lanes of
@@ -408,9 +389,9 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
 }
 
 template <typename S>
-// Two CTAs per SM (at most 128 registers): the pulse problems' bases then
-// fit one pass of the grid, which the register cache of the rows needs.
-__global__ void __launch_bounds__(CNT, 2) k_adjoint_coop(const CoopAdj<S> P) {
+// At most 128 registers: the pulse problems' bases then fit one pass of the
+// grid, which the register cache of the rows needs.
+__global__ void __launch_bounds__(CNT, 1) k_adjoint_coop(const CoopAdj<S> P) {
   __shared__ double red[2 * (CNT / 32)];
   __shared__ double s_ov[2];
   const int64_t dim = P.B.dim;

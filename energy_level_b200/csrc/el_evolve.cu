@@ -107,6 +107,12 @@ extern "C" int el_cheb_step(el_ctx *ctx, el_ham *h, int dtype, void *psi,
   if (rc) return rc;
   const double a = plan.a, b = plan.b;
   const int M = plan.M;
+  if (el::cheb_coop_ok(ctx, h, dtype, psi, M)) {
+    rc = el::cheb_coop(ctx, h, dtype, psi, plan);
+    if (rc) return rc;
+    if (n_terms) *n_terms = M + 1;
+    return EL_OK;
+  }
   auto coef = [&](int m, double *re, double *im) { *re = plan.c_re[m]; *im = plan.c_im[m]; };
   char *buf = (char *)el::workspace(ctx, 5, 4 * vb);
   if (!buf) return EL_ENOMEM;

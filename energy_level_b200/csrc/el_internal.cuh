@@ -368,6 +368,10 @@ int cheb_plan(el_ctx *ctx, el_ham *h, double tau_ns, double tol, ChebPlan *plan)
 // The expansion for a spectrum inside [lo, hi] (what cheb_plan does after
 // its Gershgorin bound).
 void cheb_plan_bounds(double lo, double hi, double tau_ns, double tol, ChebPlan *plan);
+// A whole Chebyshev step on a small full basis as one cooperative launch
+// (el_cheb_coop.cu).
+bool cheb_coop_ok(const el_ctx *ctx, const el_ham *h, int dtype, const void *psi, int M);
+int cheb_coop(el_ctx *ctx, el_ham *h, int dtype, void *psi, const ChebPlan &plan);
 // The whole adjoint gradient as one cooperative launch (el_adjoint_coop.cu):
 // vectors in buf (K+1 checkpoints, Mmax+1 terms -- of every step if stored --,
 // 3 adjoint vectors, lambda), per-step dots into hg, the objective into F.
