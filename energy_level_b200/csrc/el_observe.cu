@@ -24,6 +24,7 @@
 // in a fixed order (deterministic results).
 #include "el_internal.cuh"
 
+#include <algorithm>
 #include <vector>
 
 namespace {
@@ -139,11 +140,199 @@ __global__ void __launch_bounds__(256, 2) k_obs_items(BasisDev B, const S *__res
   }
 }
 
-__global__ void k_obs_sum(int nparts, int K, const double *__restrict__ partials, double *__restrict__ out) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < nparts; ++b) s += partials[(size_t)b * K + k];
+// out[k] = sum over the blocks' partials: 32 outputs per block, 8 threads
+// each (a fixed order).
+__global__ void __launch_bounds__(256) k_obs_sum(int nparts, int K, const double *__restrict__ partials,
+                                                 double *__restrict__ out) {
+  __shared__ double red[8][32];
+  const int k = blockIdx.x * 32 + (threadIdx.x & 31), sh = threadIdx.x >> 5;
+  double s = 0.0;
+  if (k < K) {
+#pragma unroll 8
+    for (int b = sh; b < nparts; b += 8) s += partials[(size_t)b * K + k];
+  }
+  red[sh][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (sh == 0 && k < K) {
+    for (int w = 1; w < 8; ++w) s += red[w][threadIdx.x];
     out[k] = s;
+  }
+}
+
+// ------------------------------------------- sites and all pairs at once
+// Norm, <n_i> and <sigma-_i> of every site or, with PAIRS, <n_i n_j> and
+// <sigma+_i sigma-_j> of every pair i < j, on bases of at most 32 sites (two
+// launches: both sets of sums together do not fit the registers).  For
+// a row u let a_k = v_{u + k} where site k can be excited from u, else 0; then
+//     <sigma-_k> = sum_u conj(v_u) a_k,  <sigma+_i sigma-_j> = sum_u conj(a_i) a_j,
+// so the flip targets of a row are found once for all pairs (an item per pair
+// finds two per row): the pair sums are a Gram matrix of the a_k.  A CTA
+// stages 256 rows (128 with PAIRS): codes and amplitudes, then the a_k (a
+// thread has every 64th row and a group of 8 sites; site sums in registers,
+// a_k of pairs in shared memory), then 36
+// blocks of 4 x 4 sites (i-block <= j-block), each shared by 7 threads with
+// their share of the rows, add their 16 pairs in FP64 registers.  Bound: FP64
+// multiply-adds (4 per pair and row).  31-site chain (dim 3,524,578,
+// complex64), 465 pairs: 13.7 ms with an item per pair, 2.1 here; sites
+// alone 0.83 -> 0.52 ms.
+constexpr int obs_rows(bool pairs) { return pairs ? 128 : 256; }   // rows per stage
+constexpr int OB = 8;             // blocks of 4 sites
+constexpr int OT = OB * (OB + 1) / 2;   // site-block pairs
+constexpr int OSL = 256 / OT;     // threads (row shares) of a site-block pair
+
+template <typename S, bool C, bool PAIRS>
+__global__ void __launch_bounds__(256, 2) k_obs_all(BasisDev B, const S *__restrict__ psi,
+                                                    double *__restrict__ partials, int K) {
+  constexpr int SITES = 32, OR = obs_rows(PAIRS);
+  __shared__ uint32_t code_s[OR];
+  __shared__ double p_s[OR];
+  __shared__ S vr_s[OR], vi_s[C ? OR : 1];
+  extern __shared__ __align__(16) unsigned char obs_smem[];
+  // a_k: [site][row] (re, then im), one row of padding against bank conflicts
+  S *const ar = reinterpret_cast<S *>(obs_smem);
+  S *const ai = ar + SITES * (OR + 1);
+  const int tid = threadIdx.x, n = B.n;
+  const int g = tid / 64;                              // gather role: rows tid % 64 + 64 i, sites 8 g .. 8 g + 7
+  const int ti = tid / OSL, sl = tid - ti * OSL;       // Gram role: block pair, row share
+  int bi = 0, bj = 0;
+  if (PAIRS) {
+    int q = ti;
+    for (bi = 0; bi < OB && q >= OB - bi; ++bi) q -= OB - bi;
+    bj = bi + q;
+  }
+  const bool gram = PAIRS && ti < OT;
+  double sn[PAIRS ? 1 : 8], sr[PAIRS ? 1 : 8], si[PAIRS ? 1 : 8], norm = 0.0;
+#pragma unroll
+  for (int q = 0; q < (PAIRS ? 1 : 8); ++q) sn[q] = sr[q] = si[q] = 0.0;
+  double xr[PAIRS ? 16 : 1], xi[PAIRS ? 16 : 1], nn[PAIRS ? 16 : 1];
+#pragma unroll
+  for (int q = 0; q < (PAIRS ? 16 : 1); ++q) xr[q] = xi[q] = nn[q] = 0.0;
+  for (int64_t base = (int64_t)blockIdx.x * OR; base < B.dim; base += (int64_t)gridDim.x * OR) {
+    if (tid < OR) {
+      const int64_t row = base + tid;
+      uint32_t c = 0;
+      double re = 0.0, im = 0.0;
+      if (row < B.dim) {
+        c = (uint32_t)el::unrank_row(B, row);
+        load_amp<S, C>(psi, row, re, im);
+      }
+      code_s[tid] = c;
+      p_s[tid] = re * re + im * im;
+      vr_s[tid] = (S)re;
+      if constexpr (C) vi_s[tid] = (S)im;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int r = tid & 63; r < OR; r += 64) {
+      const uint32_t code = code_s[r];
+      const int64_t row = base + r;
+      const double p = p_s[r], vr = vr_s[r], vi = C ? (double)vi_s[C ? r : 0] : 0.0;
+      if (g == 0) norm += p;
+      S wr[8], wi[8];
+      bool ok[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int k = g * 8 + q;
+        wr[q] = S(0);
+        wi[q] = S(0);
+        ok[q] = false;
+        if (k < n && row < B.dim && !((code >> k) & 1u)) {
+          const int64_t t = el::flip_target(B, code, row, k);
+          if (t >= 0) {
+            ok[q] = true;
+            if constexpr (C) { wr[q] = psi[2 * t]; wi[q] = psi[2 * t + 1]; }
+            else { wr[q] = psi[t]; }
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int k = g * 8 + q;
+        if constexpr (PAIRS) {
+          ar[k * (OR + 1) + r] = wr[q];
+          if constexpr (C) ai[k * (OR + 1) + r] = wi[q];
+        } else {
+          if ((code >> k) & 1u) sn[q] += p;
+          if (ok[q]) {
+            const double dr = wr[q], di = wi[q];
+            sr[q] += vr * dr + vi * di;      // conj(v_u) a_k
+            si[q] += vr * di - vi * dr;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (gram) {
+      for (int u = sl; u < OR; u += OSL) {
+        const uint32_t code = code_s[u];
+        const double p = p_s[u];
+        double ir[4], ii[4], jr[4], ji[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          ir[q] = ar[(bi * 4 + q) * (OR + 1) + u];
+          jr[q] = ar[(bj * 4 + q) * (OR + 1) + u];
+          ii[q] = C ? (double)ai[(bi * 4 + q) * (OR + 1) + u] : 0.0;
+          ji[q] = C ? (double)ai[(bj * 4 + q) * (OR + 1) + u] : 0.0;
+        }
+        const uint32_t mi = code >> (bi * 4), mj = code >> (bj * 4);
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            xr[x * 4 + y] += ir[x] * jr[y] + ii[x] * ji[y];    // conj(a_i) a_j
+            if constexpr (C) xi[x * 4 + y] += ir[x] * ji[y] - ii[x] * jr[y];
+            if ((mi >> x) & (mj >> y) & 1u) nn[x * 4 + y] += p;
+          }
+      }
+    }
+    __syncthreads();
+  }
+  // block sums in fixed orders, through shared memory
+  double *const red = reinterpret_cast<double *>(obs_smem);
+  double *const out = partials + (size_t)blockIdx.x * K;
+  if constexpr (!PAIRS) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        sn[q] += __shfl_xor_sync(0xffffffffu, sn[q], o);
+        sr[q] += __shfl_xor_sync(0xffffffffu, sr[q], o);
+        si[q] += __shfl_xor_sync(0xffffffffu, si[q], o);
+      }
+    for (int o = 16; o > 0; o >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, o);
+    const int warp = tid >> 5;               // warps 2 g and 2 g + 1 hold group g
+    if ((tid & 31) == 0) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        red[(warp * 8 + q) * 3] = sn[q];
+        red[(warp * 8 + q) * 3 + 1] = sr[q];
+        red[(warp * 8 + q) * 3 + 2] = si[q];
+      }
+      red[192 + warp] = norm;
+    }
+    __syncthreads();
+    if (tid == 0) out[0] = red[192] + red[193];
+    for (int o = tid; o < 3 * n; o += 256) {
+      const int k = o / 3, c = o - 3 * k, w = 2 * (k / 8);
+      out[1 + o] = red[(w * 8 + k % 8) * 3 + c] + red[((w + 1) * 8 + k % 8) * 3 + c];
+    }
+  }
+  if constexpr (PAIRS) {
+    // [bit i][bit j] of (nn, re, im), one quantity at a time
+    for (int c = 0; c < 3; ++c) {
+      __syncthreads();
+      if (gram) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) red[(size_t)tid * 16 + q] = c == 0 ? nn[q] : c == 1 ? xr[q] : xi[q];
+      }
+      __syncthreads();
+      for (int o = tid; o < OT * 16; o += 256) {
+        const int b = o / 16, q = o - 16 * b;
+        double sum = 0.0;
+        for (int w = 0; w < OSL; ++w) sum += red[(size_t)(b * OSL + w) * 16 + q];
+        out[o * 3 + c] = sum;
+      }
+    }
   }
 }
 
@@ -184,7 +373,59 @@ int run_items(el_ctx *ctx, el_ham *h, int dtype, const void *psi, std::vector<Ob
     default: return fail(ctx, EL_EINVAL, "unknown dtype %d", dtype);
   }
   EL_LAUNCH_CHECK(ctx);
-  k_obs_sum<<<(K + 255) / 256, 256, 0, ctx->stream>>>(gx, K, ctx->d_partials, d_out);
+  k_obs_sum<<<(K + 31) / 32, 256, 0, ctx->stream>>>(gx, K, ctx->d_partials, d_out);
+  EL_LAUNCH_CHECK(ctx);
+  out.assign(K, 0.0);
+  EL_CUDA_TRY(ctx, el::copy(ctx, out.data(), d_out, (size_t)K * sizeof(double), cudaMemcpyDeviceToHost));
+  EL_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  return EL_OK;
+}
+
+// Position of pair (bit i < bit j) in k_obs_all's pair sums.
+int gram_slot(int i, int j) {
+  const int bi = i / 4, bj = j / 4;
+  int b = 0;
+  for (int q = 0; q < bi; ++q) b += OB - q;
+  return (b + bj - bi) * 16 + (i % 4) * 4 + j % 4;
+}
+
+template <typename S, bool C, bool PAIRS>
+int launch_obs_all(el_ctx *ctx, const BasisDev &B, const void *psi, int gx, int K) {
+  size_t smem = 256 * sizeof(double);      // block sums of the sites
+  if (PAIRS) smem = std::max((size_t)32 * (obs_rows(true) + 1) * sizeof(S) * (C ? 2 : 1), (size_t)256 * 16 * sizeof(double));
+  auto *fn = k_obs_all<S, C, PAIRS>;
+  if (smem > 48 * 1024)
+    EL_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  fn<<<gx, 256, smem, ctx->stream>>>(B, (const S *)psi, ctx->d_partials, K);
+  EL_LAUNCH_CHECK(ctx);
+  return EL_OK;
+}
+
+template <bool PAIRS>
+int launch_obs_dtype(el_ctx *ctx, const BasisDev &B, int dtype, const void *psi, int gx, int K) {
+  switch (dtype) {
+    case EL_F32: return launch_obs_all<float, false, PAIRS>(ctx, B, psi, gx, K);
+    case EL_F64: return launch_obs_all<double, false, PAIRS>(ctx, B, psi, gx, K);
+    case EL_C64: return launch_obs_all<float, true, PAIRS>(ctx, B, psi, gx, K);
+    case EL_C128: return launch_obs_all<double, true, PAIRS>(ctx, B, psi, gx, K);
+    default: return fail(ctx, EL_EINVAL, "unknown dtype %d", dtype);
+  }
+}
+
+// out: norm, then (n, Re sm, Im sm) per bit position; or with pairs the
+// (nn, Re, Im) sums of k_obs_all.
+int run_all(el_ctx *ctx, el_ham *h, int dtype, const void *psi, bool pairs, std::vector<double> &out) {
+  const BasisDev B = el::basis_dev(h->basis);
+  const int K = pairs ? OT * 16 * 3 : 1 + 3 * B.n;
+  const int64_t stages = (B.dim + obs_rows(pairs) - 1) / obs_rows(pairs);
+  const int gx = (int)std::min<int64_t>(stages, 2 * (int64_t)el::sm_count(ctx));
+  double *d_out = (double *)el::workspace(ctx, 10, (size_t)K * sizeof(double));
+  if (!d_out) return EL_ENOMEM;
+  int rc = el::ensure_partials(ctx, (size_t)gx * K);
+  if (rc) return rc;
+  rc = pairs ? launch_obs_dtype<true>(ctx, B, dtype, psi, gx, K) : launch_obs_dtype<false>(ctx, B, dtype, psi, gx, K);
+  if (rc) return rc;
+  k_obs_sum<<<(K + 31) / 32, 256, 0, ctx->stream>>>(gx, K, ctx->d_partials, d_out);
   EL_LAUNCH_CHECK(ctx);
   out.assign(K, 0.0);
   EL_CUDA_TRY(ctx, el::copy(ctx, out.data(), d_out, (size_t)K * sizeof(double), cudaMemcpyDeviceToHost));
@@ -202,6 +443,35 @@ extern "C" int el_spin_observables(el_ctx *ctx, el_ham *h, int dtype, const void
   const int n = h->n;
   if (n_pairs < 0 || (n_pairs > 0 && (!pi || !pj))) return fail(ctx, EL_EINVAL, "bad pair list");
   EL_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+  // every site, and every pair when about as many are wanted as one Gram pass
+  // costs (it takes the time of 36 pair items: 31-site chain, 6 groups)
+  // (not the pairs of a fixed-excitation sector: the row with both sites
+  // clear, from which the Gram matrix starts, is outside it)
+  if (n <= 32 && (n_pairs == 0 || (n_pairs >= 36 && h->basis->kind != EL_BASIS_CHARGE))) {
+    for (int p = 0; p < n_pairs; ++p)
+      if (pi[p] < 0 || pj[p] < 0 || pi[p] >= n || pj[p] >= n || pi[p] == pj[p])
+        return fail(ctx, EL_EINVAL, "pair %d: bad sites (%d, %d)", p, pi[p], pj[p]);
+    std::vector<double> out;
+    int rc = run_all(ctx, h, dtype, psi, false, out);
+    if (rc) return rc;
+    if (norm) *norm = out[0];
+    for (int i = 0; i < n; ++i) {
+      const double *o = &out[1 + 3 * (n - 1 - i)];
+      if (n_site) n_site[i] = o[0];
+      if (sigma_minus) { sigma_minus[2 * i] = o[1]; sigma_minus[2 * i + 1] = o[2]; }
+    }
+    if (n_pairs > 0) {
+      rc = run_all(ctx, h, dtype, psi, true, out);
+      if (rc) return rc;
+    }
+    for (int p = 0; p < n_pairs; ++p) {
+      const int bi = n - 1 - pi[p], bj = n - 1 - pj[p];
+      const double *o = &out[3 * (size_t)gram_slot(std::min(bi, bj), std::max(bi, bj))];
+      if (nn) nn[p] = o[0];
+      if (xy) { xy[2 * p] = o[1]; xy[2 * p + 1] = bi < bj ? o[2] : -o[2]; }   // conj(a_i) a_j
+    }
+    return EL_OK;
+  }
   std::vector<ObsItem> items;
   items.push_back(item(kNormItem, 0, 0));
   for (int i = 0; i < n; ++i) items.push_back(item(kSiteItem, n - 1 - i, 0));

@@ -164,16 +164,6 @@ def _start_state(psi0, n, codes, dim, dtype, device):
     return torch.as_tensor(state_vector(psi0, n, codes), dtype=dtype, device=device).contiguous()
 
 
-def _host_amplitudes(psi, step=1 << 24):
-    """The state as a complex128 numpy array, widened on the device in pieces."""
-    import torch
-    out = np.empty(psi.numel(), np.complex128)
-    to = torch.from_numpy(out)
-    for lo in range(0, psi.numel(), step):
-        to[lo:lo + step].copy_(psi[lo:lo + step].to(torch.complex128))
-    return out
-
-
 def evolve_manybody(calib, psi0=None, t_grid=None, Om=None, delta=None, gamma=None, terms=None,
                     segments=None, progress_arr=None, log=None, want_corr=True, want_entropy=True,
                     max_dim=None, entropy_cut=None, record_psi=False, diag=False, plan=None,
@@ -357,5 +347,5 @@ def evolve_manybody(calib, psi0=None, t_grid=None, Om=None, delta=None, gamma=No
         diag=({'dim': dim, 'n_atoms': n, 'backend': backend, 'launches': ctx.launches} if diag else None),
         observables=obs)
     if record_psi:
-        out['psi_amp'] = _host_amplitudes(psi)
+        out['psi_amp'] = psi.cpu().numpy().astype(np.complex128)
     return out
