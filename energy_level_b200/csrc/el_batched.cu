@@ -47,7 +47,8 @@ struct BatchArgs {
   const Inst *inst;             // [count], processing order
   const double *diag;           // concatenated diagonal (FP64)
   void *ws;                     // per-CTA workspace: (max_iter + 2) * dim_max values
-  int64_t dim_max;
+  int64_t dim_max;              // rows from one workspace vector to the next (16-byte multiple)
+  int64_t smem_rows;            // instances up to this size keep the current vector in shared memory
   unsigned int *queue;
   uint64_t seed;
   double *e0, *e1, *res, *gap;  // outputs in processing order
@@ -236,8 +237,179 @@ __device__ __forceinline__ int64_t flip_b(const Inst &I, const uint64_t *fib, ui
   return set ? row - w : row + w;
 }
 
+// H v on rows r0, r0 + NT, .. of an instance (4 rows of this thread), the sum
+// in ascending bit order.  x: the vector, in shared memory where it fits.  The
+// bit loop is uniform over the CTA, so a bit's amplitude and weight are read
+// once for 4 rows, and codes, ranks and targets are 32-bit; bases of more than
+// 32 sites take the 64-bit targets bit by bit.
+constexpr int HR = 4;
+
+template <typename T, int NT>
+__device__ __forceinline__ void batch_hv(const Inst &I, const uint64_t *fib, const double *D, const T *x,
+                                         int64_t r0, double (&h)[HR]) {
+  const int n = I.n, lay = I.layout;
+  const int64_t dim = I.dim;
+  bool on[HR];
+#pragma unroll
+  for (int i = 0; i < HR; ++i) {
+    on[i] = r0 + i * NT < dim;
+    h[i] = on[i] ? D[r0 + i * NT] * (double)x[r0 + i * NT] : 0.0;
+  }
+  if (n <= 32 && lay != EL_LAYOUT_TABLE) {
+    const uint32_t full = n == 32 ? 0xffffffffu : (1u << n) - 1u;
+    uint32_t code[HR], flips[HR];
+#pragma unroll
+    for (int i = 0; i < HR; ++i) {
+      code[i] = on[i] ? (uint32_t)unrank_b(I, fib, r0 + i * NT) : 0u;
+      flips[i] = full;
+      if (lay != EL_LAYOUT_FULL) {
+        uint32_t near = (code[i] << 1) | (code[i] >> 1);
+        if (lay == EL_LAYOUT_RING) near |= ((code[i] >> (n - 1)) & 1u) | ((code[i] & 1u) << (n - 1));
+        flips[i] = code[i] | (~near & full);
+      }
+      if (!on[i]) flips[i] = 0u;
+    }
+    const int top = lay == EL_LAYOUT_RING ? n - 1 : n;      // ring: the top bit's target below
+    for (int k = 0; k < top; ++k) {
+      const double amp = I.om[k];
+      if (amp == 0.0) continue;
+      const int w = lay == EL_LAYOUT_FULL ? 1 << k : (int)fib[k + 2];
+      const int w1 = lay == EL_LAYOUT_RING ? (int)fib[k + 1] : w;   // weight with the ring's top bit set
+      T xv[HR];
+#pragma unroll
+      for (int i = 0; i < HR; ++i) {
+        const int wi = (lay == EL_LAYOUT_RING && ((code[i] >> (n - 1)) & 1u)) ? w1 : w;
+        const int r = (int)r0 + i * NT;
+        const int t = ((code[i] >> k) & 1u) ? r - wi : r + wi;
+        if ((flips[i] >> k) & 1u) xv[i] = x[t];
+      }
+#pragma unroll
+      for (int i = 0; i < HR; ++i)
+        if ((flips[i] >> k) & 1u) h[i] += amp * (double)xv[i];
+    }
+    if (top < n && I.om[n - 1] != 0.0) {
+#pragma unroll
+      for (int i = 0; i < HR; ++i)
+        if ((flips[i] >> (n - 1)) & 1u)
+          h[i] += I.om[n - 1] * (double)x[ring_rank(fib, n, (uint64_t)(code[i] ^ (1u << (n - 1))))];
+    }
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < HR; ++i) {
+    if (!on[i]) continue;
+    const int64_t r = r0 + i * NT;
+    const uint64_t code = unrank_b(I, fib, r);
+    for (int k = 0; k < n; ++k) {
+      const double amp = I.om[k];
+      if (amp == 0.0) continue;
+      const int64_t t = flip_b(I, fib, code, r, k);
+      if (t >= 0) h[i] += amp * (double)x[t];
+    }
+  }
+}
+
+// 16-byte pieces of a vector (workspace rows start on 16-byte boundaries).
+template <typename T> struct alignas(16) Piece {
+  static constexpr int W = 16 / (int)sizeof(T);
+  T v[W];
+};
+
+// cf[q] = <v_sel[q], w> for the ns selected vectors.  Groups of GQ vectors
+// share the read of w, every thread has GQ + 1 16-byte loads in flight, and a
+// group's sums are reduced together.
+template <typename T, int NT>
+__device__ void batch_dots(const T *Vb, int64_t ld, const T *W, int64_t dim, const short *sel, int ns,
+                           double (*red2)[8], double *cf) {
+  constexpr int GQ = NT >= 1024 ? 4 : 8;
+  typedef Piece<T> P;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t np = dim / P::W;
+  for (int q0 = 0; q0 < ns; q0 += GQ) {
+    const T *vk[GQ];
+    double acc[GQ];
+#pragma unroll
+    for (int q = 0; q < GQ; ++q) {
+      vk[q] = Vb + (size_t)sel[min(q0 + q, ns - 1)] * ld;
+      acc[q] = 0.0;
+    }
+    for (int64_t c = tid; c < np; c += NT) {
+      const P w = reinterpret_cast<const P *>(W)[c];
+      P v[GQ];
+#pragma unroll
+      for (int q = 0; q < GQ; ++q) v[q] = reinterpret_cast<const P *>(vk[q])[c];
+#pragma unroll
+      for (int q = 0; q < GQ; ++q)
+#pragma unroll
+        for (int e = 0; e < P::W; ++e) acc[q] += (double)v[q].v[e] * (double)w.v[e];
+    }
+    for (int64_t r = np * P::W + tid; r < dim; r += NT)
+#pragma unroll
+      for (int q = 0; q < GQ; ++q) acc[q] += (double)vk[q][r] * (double)W[r];
+#pragma unroll
+    for (int q = 0; q < GQ; ++q)
+      for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    __syncthreads();            // the previous group's sums are read
+    if (lane == 0) {
+#pragma unroll
+      for (int q = 0; q < GQ; ++q) red2[warp][q] = acc[q];
+    }
+    __syncthreads();
+    if (tid < GQ && q0 + tid < ns) {
+      double s = 0.0;
+      for (int w = 0; w < NT / 32; ++w) s += red2[w][tid];
+      cf[q0 + tid] = s;
+    }
+  }
+  __syncthreads();
+}
+
+// w -= sum_q cf[q] v_sel[q]; returns this thread's part of |w|^2.
+template <typename T, int NT>
+__device__ double batch_subtract(const T *Vb, int64_t ld, T *W, int64_t dim, const short *sel, int ns,
+                                 const double *cf) {
+  typedef Piece<T> P;
+  const int tid = threadIdx.x;
+  const int64_t np = dim / P::W;
+  double n2 = 0.0;
+  for (int64_t c = tid; c < np; c += NT) {
+    const P w = reinterpret_cast<const P *>(W)[c];
+    double s[P::W];
+#pragma unroll
+    for (int e = 0; e < P::W; ++e) s[e] = 0.0;
+#pragma unroll 8
+    for (int q = 0; q < ns; ++q) {
+      const P v = reinterpret_cast<const P *>(Vb + (size_t)sel[q] * ld)[c];
+      const double a = cf[q];
+#pragma unroll
+      for (int e = 0; e < P::W; ++e) s[e] += a * (double)v.v[e];
+    }
+    P o;
+#pragma unroll
+    for (int e = 0; e < P::W; ++e) {
+      o.v[e] = (T)((double)w.v[e] - s[e]);
+      n2 += (double)o.v[e] * (double)o.v[e];
+    }
+    reinterpret_cast<P *>(W)[c] = o;
+  }
+  for (int64_t r = np * P::W + tid; r < dim; r += NT) {
+    double s = 0.0;
+    for (int q = 0; q < ns; ++q) s += cf[q] * (double)Vb[(size_t)sel[q] * ld + r];
+    const T o = (T)((double)W[r] - s);
+    n2 += (double)o * (double)o;
+    W[r] = o;
+  }
+  return n2;
+}
+
+// The current vector of an instance of up to smem_rows rows is held in
+// dynamic shared memory, where the flips of every row gather it; its rows are
+// read from L2 otherwise.
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_lanczos_batch(const BatchArgs A) {
+  extern __shared__ __align__(16) unsigned char batch_smem[];
+  T *const vs = reinterpret_cast<T *>(batch_smem);
+  __shared__ double red2[NT / 32][8];
   __shared__ Inst I;
   __shared__ uint64_t fib[MAXN + 3];
   __shared__ double red[NT / 32];
@@ -278,9 +450,14 @@ __global__ void __launch_bounds__(NT) k_lanczos_batch(const BatchArgs A) {
       nrm += (double)v * (double)v;
     }
     nrm = block_sum<NT>(nrm, red);
+    const bool shared = dim <= A.smem_rows;
     {
       const T sc = (T)(1.0 / sqrt(nrm));
-      for (int64_t r = tid; r < dim; r += NT) Vb[r] *= sc;
+      for (int64_t r = tid; r < dim; r += NT) {
+        const T v = Vb[r] * sc;
+        Vb[r] = v;
+        if (shared) vs[r] = v;
+      }
     }
     if (tid == 0) {
       wcur[0] = 1.0; s_force = 0; s_done = 0; s_th[0] = s_th[1] = 0.0; s_res[0] = s_res[1] = 1e300;
@@ -294,23 +471,24 @@ __global__ void __launch_bounds__(NT) k_lanczos_batch(const BatchArgs A) {
       const T *vp = j ? Vb + (size_t)(j - 1) * A.dim_max : nullptr;
       // w = H v - beta v_prev ; alpha = <v, w>
       double pa = 0.0;
-      for (int64_t r = tid; r < dim; r += NT) {
-        const uint64_t code = unrank_b(I, fib, r);
-        double h = D[r] * (double)v[r];
-        for (int k = 0; k < I.n; ++k) {
-          const double amp = I.om[k];
-          if (amp == 0.0) continue;
-          const int64_t t = flip_b(I, fib, code, r, k);
-          if (t >= 0) h += amp * (double)v[t];
+      const T *x = shared ? vs : v;
+      for (int64_t r0 = tid; r0 < dim; r0 += (int64_t)HR * NT) {
+        double h[HR];
+        batch_hv<T, NT>(I, fib, D, x, r0, h);
+#pragma unroll
+        for (int i = 0; i < HR; ++i) {
+          const int64_t r = r0 + i * NT;
+          if (r >= dim) break;
+          const T wv = (T)(h[i] - (vp ? beta * (double)vp[r] : 0.0));
+          W[r] = wv;
+          pa += (double)x[r] * (double)wv;
         }
-        const T wv = (T)(h - (vp ? beta * (double)vp[r] : 0.0));
-        W[r] = wv;
-        pa += (double)v[r] * (double)wv;
       }
       const double alpha = block_sum<NT>(pa, red);
       double pn = 0.0;
+#pragma unroll 4
       for (int64_t r = tid; r < dim; r += NT) {
-        const T wv = (T)((double)W[r] - alpha * (double)v[r]);
+        const T wv = (T)((double)W[r] - alpha * (double)x[r]);
         W[r] = wv;
         pn += (double)wv * (double)wv;
       }
@@ -360,50 +538,14 @@ __global__ void __launch_bounds__(NT) k_lanczos_batch(const BatchArgs A) {
       }
       __syncthreads();
       if (s_flag && j > 0) {
-        // classical Gram-Schmidt, twice: each warp forms the dot products of
-        // its share of v_0..v_j with w (FP64, fixed order), then every thread
-        // subtracts all projections from its rows
+        // classical Gram-Schmidt, twice
         double *cf = work + 2 * MAXIT;
+        double pn2 = 0.0;
         for (int pass = 0; pass < 2; ++pass) {
-          const int lane = tid & 31, warp = tid >> 5;
-          const int ns = nsel;
-          for (int q = warp; q < ns; q += NT / 32) {
-            const T *vk = Vb + (size_t)sel[q] * A.dim_max;
-            double pc0 = 0.0, pc1 = 0.0, pc2 = 0.0, pc3 = 0.0;
-            int64_t r = lane;
-            for (; r + 96 < dim; r += 128) {
-              pc0 += (double)vk[r] * (double)W[r];
-              pc1 += (double)vk[r + 32] * (double)W[r + 32];
-              pc2 += (double)vk[r + 64] * (double)W[r + 64];
-              pc3 += (double)vk[r + 96] * (double)W[r + 96];
-            }
-            for (; r < dim; r += 32) pc0 += (double)vk[r] * (double)W[r];
-            double pc = (pc0 + pc1) + (pc2 + pc3);
-            for (int o = 16; o > 0; o >>= 1) pc += __shfl_xor_sync(0xffffffffu, pc, o);
-            if (lane == 0) cf[q] = pc;
-          }
-          __syncthreads();
-          for (int64_t r = tid; r < dim; r += NT) {
-            const T *col = Vb + r;
-            double w0 = (double)W[r], w1 = 0.0, w2 = 0.0, w3 = 0.0;
-            int q = 0;
-            for (; q + 4 <= ns; q += 4) {
-              const double v0 = (double)col[(size_t)sel[q] * A.dim_max];
-              const double v1 = (double)col[(size_t)sel[q + 1] * A.dim_max];
-              const double v2 = (double)col[(size_t)sel[q + 2] * A.dim_max];
-              const double v3 = (double)col[(size_t)sel[q + 3] * A.dim_max];
-              w0 -= cf[q] * v0;
-              w1 -= cf[q + 1] * v1;
-              w2 -= cf[q + 2] * v2;
-              w3 -= cf[q + 3] * v3;
-            }
-            for (; q < ns; ++q) w0 -= cf[q] * (double)col[(size_t)sel[q] * A.dim_max];
-            W[r] = (T)((w0 + w1) + (w2 + w3));
-          }
+          batch_dots<T, NT>(Vb, A.dim_max, W, dim, sel, nsel, red2, cf);
+          pn2 = batch_subtract<T, NT>(Vb, A.dim_max, W, dim, sel, nsel, cf);
           __syncthreads();
         }
-        double pn2 = 0.0;
-        for (int64_t r = tid; r < dim; r += NT) pn2 += (double)W[r] * (double)W[r];
         b2 = block_sum<NT>(pn2, red);
         bnext = sqrt(fmax(b2, 0.0));
       }
@@ -475,7 +617,12 @@ __global__ void __launch_bounds__(NT) k_lanczos_batch(const BatchArgs A) {
       // v_{j+1} = w / beta
       T *vn = Vb + (size_t)(j + 1) * A.dim_max;
       const double inv = 1.0 / bnext;
-      for (int64_t r = tid; r < dim; r += NT) vn[r] = (T)((double)W[r] * inv);
+#pragma unroll 4
+      for (int64_t r = tid; r < dim; r += NT) {
+        const T v = (T)((double)W[r] * inv);
+        vn[r] = v;
+        if (shared) vs[r] = v;
+      }
       beta = bnext;
       __syncthreads();
     }
@@ -1180,7 +1327,8 @@ int el_batch_run(el_ctx *ctx, el_batch *b, int threads, int ctas_per_sm, uint64_
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const int grid = std::min(b->count, sms * ctas_per_sm);
   const size_t es = b->dtype == EL_F32 ? 4 : 8;
-  const size_t need = (size_t)grid * (b->max_iter + 2) * b->dim_max * es;
+  const int64_t ld = (b->dim_max + 3) / 4 * 4;
+  const size_t need = (size_t)grid * (b->max_iter + 2) * ld * es;
   if (need > b->ws_bytes) {
     // grows only outside graph capture (a first run sizes it)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1198,18 +1346,37 @@ int el_batch_run(el_ctx *ctx, el_batch *b, int threads, int ctas_per_sm, uint64_
   BatchArgs A;
   memset(&A, 0, sizeof A);
   A.count = b->count; A.max_iter = b->max_iter; A.tol = b->tol; A.eps = b->dtype == EL_F32 ? 1.19e-7 : 2.22e-16;
-  A.inst = b->d_inst; A.diag = b->d_diag; A.ws = b->ws; A.dim_max = b->dim_max; A.queue = b->d_queue;
+  A.inst = b->d_inst; A.diag = b->d_diag; A.ws = b->ws; A.dim_max = ld; A.queue = b->d_queue;
   A.seed = seed;
   A.e0 = b->d_out; A.e1 = b->d_out + b->count; A.res = b->d_out + 2 * b->count; A.gap = b->d_out + 3 * b->count;
   A.iters = b->d_iout; A.conv = b->d_iout + b->count;
   A.nat = b->want_nat ? b->d_nat : nullptr;
-#define EL_BCASE(TT, NTV) k_lanczos_batch<TT, NTV><<<grid, NTV, 0, ctx->stream>>>(A)
+  // shared memory for the largest vector, or what the CTAs of an SM leave
+  int smem_sm = 0, smem_block = 0;
+  EL_CUDA_TRY(ctx, cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
+  EL_CUDA_TRY(ctx, cudaDeviceGetAttribute(&smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  auto launch = [&](const void *fn) -> int {
+    cudaFuncAttributes fa;
+    EL_CUDA_TRY(ctx, cudaFuncGetAttributes(&fa, fn));
+    // 1 KB per CTA is the system's
+    const int64_t room = std::min<int64_t>(smem_sm / ctas_per_sm - 1024, smem_block) - (int64_t)fa.sharedSizeBytes;
+    const int64_t rows = std::max<int64_t>(0, std::min<int64_t>(room / (int64_t)es, b->dim_max));
+    A.smem_rows = rows;
+    const size_t smem = (size_t)rows * es;
+    EL_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    void *kargs[] = {(void *)&A};
+    EL_CUDA_TRY(ctx, cudaLaunchKernel(fn, dim3(grid), dim3(threads), kargs, smem, ctx->stream));
+    return EL_OK;
+  };
+  int lrc = EL_OK;
+#define EL_BCASE(TT, NTV) lrc = launch((const void *)k_lanczos_batch<TT, NTV>)
   if (b->dtype == EL_F32) {
     if (threads == 256) EL_BCASE(float, 256); else if (threads == 512) EL_BCASE(float, 512); else EL_BCASE(float, 1024);
   } else {
     if (threads == 256) EL_BCASE(double, 256); else if (threads == 512) EL_BCASE(double, 512); else EL_BCASE(double, 1024);
   }
 #undef EL_BCASE
+  if (lrc) return lrc;
   EL_LAUNCH_CHECK(ctx);
   return EL_OK;
 }
