@@ -237,15 +237,40 @@ __device__ __forceinline__ int64_t flip_b(const Inst &I, const uint64_t *fib, ui
   return set ? row - w : row + w;
 }
 
-// H v on rows r0, r0 + NT, .. of an instance (4 rows of this thread), the sum
-// in ascending bit order.  x: the vector, in shared memory where it fits.  The
+// What H v reads of a row before its flips: diagonal, code, previous vector.
+// Four rows per thread (NT apart); the next four are read while the current
+// four are worked on, since 16 warps do not cover the reads' latency.
+constexpr int HR = 4;
+
+template <typename T> struct RowsIn {
+  double d[HR];
+  uint64_t code[HR];
+  T vp[HR];
+};
+
+template <typename T, int NT>
+__device__ __forceinline__ void batch_rows(const Inst &I, const uint64_t *fib, const double *D, const T *vp,
+                                           int64_t r0, RowsIn<T> &R) {
+#pragma unroll
+  for (int i = 0; i < HR; ++i) {
+    const int64_t r = r0 + i * NT;
+    R.d[i] = 0.0;
+    R.code[i] = 0;
+    R.vp[i] = T(0);
+    if (r >= I.dim) continue;
+    R.d[i] = D[r];
+    R.code[i] = unrank_b(I, fib, r);
+    if (vp) R.vp[i] = vp[r];
+  }
+}
+
+// h = H v on rows r0, r0 + NT, .. (4 rows of this thread), the sum in
+// ascending bit order.  x: the vector, in shared memory where it fits.  The
 // bit loop is uniform over the CTA, so a bit's amplitude and weight are read
 // once for 4 rows, and codes, ranks and targets are 32-bit; bases of more than
 // 32 sites take the 64-bit targets bit by bit.
-constexpr int HR = 4;
-
 template <typename T, int NT>
-__device__ __forceinline__ void batch_hv(const Inst &I, const uint64_t *fib, const double *D, const T *x,
+__device__ __forceinline__ void batch_hv(const Inst &I, const uint64_t *fib, const RowsIn<T> &R, const T *x,
                                          int64_t r0, double (&h)[HR]) {
   const int n = I.n, lay = I.layout;
   const int64_t dim = I.dim;
@@ -253,14 +278,14 @@ __device__ __forceinline__ void batch_hv(const Inst &I, const uint64_t *fib, con
 #pragma unroll
   for (int i = 0; i < HR; ++i) {
     on[i] = r0 + i * NT < dim;
-    h[i] = on[i] ? D[r0 + i * NT] * (double)x[r0 + i * NT] : 0.0;
+    h[i] = on[i] ? R.d[i] * (double)x[r0 + i * NT] : 0.0;
   }
   if (n <= 32 && lay != EL_LAYOUT_TABLE) {
     const uint32_t full = n == 32 ? 0xffffffffu : (1u << n) - 1u;
     uint32_t code[HR], flips[HR];
 #pragma unroll
     for (int i = 0; i < HR; ++i) {
-      code[i] = on[i] ? (uint32_t)unrank_b(I, fib, r0 + i * NT) : 0u;
+      code[i] = (uint32_t)R.code[i];
       flips[i] = full;
       if (lay != EL_LAYOUT_FULL) {
         uint32_t near = (code[i] << 1) | (code[i] >> 1);
@@ -270,6 +295,7 @@ __device__ __forceinline__ void batch_hv(const Inst &I, const uint64_t *fib, con
       if (!on[i]) flips[i] = 0u;
     }
     const int top = lay == EL_LAYOUT_RING ? n - 1 : n;      // ring: the top bit's target below
+#pragma unroll 2
     for (int k = 0; k < top; ++k) {
       const double amp = I.om[k];
       if (amp == 0.0) continue;
@@ -299,11 +325,10 @@ __device__ __forceinline__ void batch_hv(const Inst &I, const uint64_t *fib, con
   for (int i = 0; i < HR; ++i) {
     if (!on[i]) continue;
     const int64_t r = r0 + i * NT;
-    const uint64_t code = unrank_b(I, fib, r);
     for (int k = 0; k < n; ++k) {
       const double amp = I.om[k];
       if (amp == 0.0) continue;
-      const int64_t t = flip_b(I, fib, code, r, k);
+      const int64_t t = flip_b(I, fib, R.code[i], r, k);
       if (t >= 0) h[i] += amp * (double)x[t];
     }
   }
@@ -471,19 +496,27 @@ __global__ void __launch_bounds__(NT) k_lanczos_batch(const BatchArgs A) {
       const T *vp = j ? Vb + (size_t)(j - 1) * A.dim_max : nullptr;
       // w = H v - beta v_prev ; alpha = <v, w>
       double pa = 0.0;
-      const T *x = shared ? vs : v;
-      for (int64_t r0 = tid; r0 < dim; r0 += (int64_t)HR * NT) {
-        double h[HR];
-        batch_hv<T, NT>(I, fib, D, x, r0, h);
+      auto product = [&](const T *x) {
+        RowsIn<T> next;
+        batch_rows<T, NT>(I, fib, D, vp, tid, next);
+        for (int64_t r0 = tid; r0 < dim; r0 += (int64_t)HR * NT) {
+          const RowsIn<T> in = next;
+          batch_rows<T, NT>(I, fib, D, vp, r0 + (int64_t)HR * NT, next);
+          double h[HR];
+          batch_hv<T, NT>(I, fib, in, x, r0, h);
 #pragma unroll
-        for (int i = 0; i < HR; ++i) {
-          const int64_t r = r0 + i * NT;
-          if (r >= dim) break;
-          const T wv = (T)(h[i] - (vp ? beta * (double)vp[r] : 0.0));
-          W[r] = wv;
-          pa += (double)x[r] * (double)wv;
+          for (int i = 0; i < HR; ++i) {
+            const int64_t r = r0 + i * NT;
+            if (r >= dim) break;
+            const T wv = (T)(h[i] - (vp ? beta * (double)in.vp[i] : 0.0));
+            W[r] = wv;
+            pa += (double)x[r] * (double)wv;
+          }
         }
-      }
+      };
+      if (shared) product(vs);   // two copies of the loop: shared-memory loads in the first
+      else product(v);
+      const T *x = shared ? vs : v;
       const double alpha = block_sum<NT>(pa, red);
       double pn = 0.0;
 #pragma unroll 4
