@@ -62,5 +62,8 @@ int launch_chain_block(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const BasisDe
 // The same on the full 2^n basis (el_full.cu).
 bool full_block_ok(const el_ham *h, const ApplyArgs &A);
 int launch_full_block(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const KArgs &K);
+// The same on blockade sectors of a graph (el_table.cu).
+bool table_block_ok(const el_ham *h, const ApplyArgs &A);
+int launch_table_block(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const BasisDev &B, const KArgs &K);
 
 }  // namespace el

@@ -159,6 +159,16 @@ int upload_tables(el_ctx *ctx, el_basis *b) {
   EL_CUDA_TRY(ctx, el::copy(ctx, b->d_pre_off, b->h_pre_off.data(), npre * sizeof(int64_t), cudaMemcpyHostToDevice));
   EL_CUDA_TRY(ctx, el::copy(ctx, b->d_pre_cls, b->h_pre_cls.data(), npre * sizeof(int32_t), cudaMemcpyHostToDevice));
   EL_CUDA_TRY(ctx, el::copy(ctx, b->d_suf_rank, b->h_suf_rank.data(), b->h_suf_rank.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+  if (b->dim < ((int64_t)1 << 31)) {
+    std::vector<int2> pack(npre);
+    for (size_t p = 0; p < npre; ++p) {
+      const bool in = b->h_pre_off[p] >= 0;
+      pack[p].x = in ? (int)b->h_pre_off[p] : -1;
+      pack[p].y = in ? b->h_pre_cls[p] : 0;
+    }
+    EL_CUDA_TRY(ctx, cudaMalloc(&b->d_pre_pack, npre * sizeof(int2)));
+    EL_CUDA_TRY(ctx, el::copy(ctx, b->d_pre_pack, pack.data(), npre * sizeof(int2), cudaMemcpyHostToDevice));
+  }
   // groups for the code expansion
   std::vector<uint64_t> gp;
   std::vector<int64_t> go;
@@ -320,6 +330,7 @@ int el_basis_destroy(el_basis *b) {
   cudaSetDevice(b->device);
   if (b->d_pre_off) cudaFree(b->d_pre_off);
   if (b->d_pre_cls) cudaFree(b->d_pre_cls);
+  if (b->d_pre_pack) cudaFree(b->d_pre_pack);
   if (b->d_suf_rank) cudaFree(b->d_suf_rank);
   if (b->d_codes) cudaFree(b->d_codes);
   delete b;

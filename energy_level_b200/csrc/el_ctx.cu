@@ -86,6 +86,7 @@ BasisDev basis_dev(const el_basis *b) {
   B.dim = b->dim;
   B.pre_off = b->d_pre_off;
   B.pre_cls = b->d_pre_cls;
+  B.pre_pack = b->d_pre_pack;
   B.suf_rank = b->d_suf_rank;
   B.codes = b->d_codes;
   for (int k = 0; k < EL_MAX_SITES; ++k) B.adj[k] = b->adj[k];

@@ -65,6 +65,7 @@ struct el_basis {
   std::vector<int64_t> h_cls_off;   // [ncls+1] offsets into h_suf_list
   int64_t *d_pre_off = nullptr;
   int32_t *d_pre_cls = nullptr;
+  int2 *d_pre_pack = nullptr;       // [2^P] (offset, class) in 32 bits, bases below 2^31 rows
   int32_t *d_suf_rank = nullptr;
   uint64_t *d_codes = nullptr;      // [dim] (TABLE layout only)
   int device = 0;
@@ -79,6 +80,7 @@ struct BasisDev {
   int64_t dim;
   const int64_t *pre_off;
   const int32_t *pre_cls;
+  const int2 *pre_pack;     // (offset or -1, class) per prefix, or null
   const int32_t *suf_rank;
   const uint64_t *codes;
   uint64_t adj[EL_MAX_SITES];
