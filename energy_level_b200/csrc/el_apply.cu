@@ -892,12 +892,13 @@ __global__ void __launch_bounds__(256) k_axpby(int64_t len, double a_re, double 
 
 // partials[bx][j] (re, im) of <V_j, w> over the block's rows.
 constexpr int GJ = 16;
-// dots_j = <V_j, w> for a group of GJ columns per blockIdx.y: every thread
-// accumulates its rows in FP64 registers, warps reduce by shuffles (fixed
+// dots_j = <V_j, w> for a group of GJ columns per blockIdx.y (200 FP64 columns
+// of 65,536 rows, L2-resident: 55 us with 8-byte loads, 14.3 with 16-byte
+// ones): every thread accumulates its rows in FP64 registers, warps reduce by shuffles (fixed
 // tree), then the block's warps in order; per-block partials are summed by
 // k_sum_partials in block order (deterministic).
-template <typename S, bool C>
-__global__ void __launch_bounds__(256) k_gemv_t(int64_t len, int k, const S *V, int64_t ld, const S *w,
+template <typename S, bool C, bool ALN>
+__global__ void __launch_bounds__(256, 2) k_gemv_t(int64_t len, int k, const S *V, int64_t ld, const S *w,
                                                 double *partials) {
   __shared__ double red[8][2 * GJ];
   const int j0 = blockIdx.y * GJ;
@@ -905,24 +906,51 @@ __global__ void __launch_bounds__(256) k_gemv_t(int64_t len, int k, const S *V, 
   double accr[GJ], acci[GJ];
 #pragma unroll
   for (int q = 0; q < GJ; ++q) { accr[q] = 0.0; acci[q] = 0.0; }
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    if constexpr (C) {
-      const double wr = w[2 * i], wi = w[2 * i + 1];
+  // E values per step: one 16-byte piece where every column starts on such a
+  // boundary (ALN), else one (complex) value
+  constexpr int E = ALN ? 16 / (int)sizeof(S) : (C ? 2 : 1);
+  struct alignas(ALN ? 16 : sizeof(S)) Chunk { S v[E]; };
+  const int64_t values = C ? 2 * len : len, cols = C ? 2 * ld : ld;
+  const int64_t chunks = values / E;
+  const S *const V0 = V + (size_t)j0 * cols;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < chunks; i += (int64_t)gridDim.x * blockDim.x) {
+    const Chunk wc = reinterpret_cast<const Chunk *>(w)[i];
+    Chunk vc[GJ];
 #pragma unroll
-      for (int q = 0; q < GJ; ++q) {
-        if (q < nq) {
-          const S *vj = V + (size_t)(j0 + q) * ld * 2;
-          const double vr = vj[2 * i], vi = vj[2 * i + 1];
+    for (int q = 0; q < GJ; ++q)
+      if (q < nq) vc[q] = reinterpret_cast<const Chunk *>(V0 + (size_t)q * cols)[i];
+#pragma unroll
+    for (int q = 0; q < GJ; ++q) {
+      if (q >= nq) continue;
+      if constexpr (C) {
+#pragma unroll
+        for (int e = 0; e < E; e += 2) {
+          const double wr = wc.v[e], wi = wc.v[e + 1], vr = vc[q].v[e], vi = vc[q].v[e + 1];
           accr[q] += vr * wr + vi * wi;
           acci[q] += vr * wi - vi * wr;
         }
-      }
-    } else {
-      const double wv = w[i];
+      } else {
 #pragma unroll
-      for (int q = 0; q < GJ; ++q)
-        if (q < nq) accr[q] += (double)V[(size_t)(j0 + q) * ld + i] * wv;
+        for (int e = 0; e < E; ++e) accr[q] += (double)vc[q].v[e] * (double)wc.v[e];
+      }
+    }
+  }
+  // values after the last piece (columns of a 16-byte pitch have fewer than E)
+  const int64_t tail0 = chunks * E;
+  if (tail0 < values && blockIdx.x == 0 && threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < GJ; ++q) {
+      if (q >= nq) continue;
+      const S *const vj = V0 + (size_t)q * cols;
+      for (int64_t t = tail0; t < values; t += C ? 2 : 1) {
+        if constexpr (C) {
+          const double wr = w[t], wi = w[t + 1], vr = vj[t], vi = vj[t + 1];
+          accr[q] += vr * wr + vi * wi;
+          acci[q] += vr * wi - vi * wr;
+        } else {
+          accr[q] += (double)vj[t] * (double)w[t];
+        }
+      }
     }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -944,19 +972,30 @@ __global__ void __launch_bounds__(256) k_gemv_t(int64_t len, int k, const S *V, 
   }
 }
 
-__global__ void k_sum_partials(int nparts, int k, const double *partials, double *out) {
-  for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < 2 * k; o += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < nparts; ++b) s += partials[(size_t)b * 2 * k + o];
+// out[o] = sum over blocks, 32 outputs per block with 8 threads each (fixed order).
+__global__ void __launch_bounds__(256) k_sum_partials(int nparts, int k, const double *partials, double *out) {
+  __shared__ double red[8][32];
+  const int o = blockIdx.x * 32 + (threadIdx.x & 31), sh = threadIdx.x >> 5;
+  double s = 0.0;
+  if (o < 2 * k) {
+#pragma unroll 4
+    for (int b = sh; b < nparts; b += 8) s += partials[(size_t)b * 2 * k + o];
+  }
+  red[sh][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (sh == 0 && o < 2 * k) {
+    for (int w = 1; w < 8; ++w) s += red[w][threadIdx.x];
     out[o] = s;
   }
 }
 
 // w -= sum_j coef_j V_j  (sub = true) or w = sum_j coef_j V_j (sub = false).
 // The coefficients are staged in shared memory (k <= GN_MAX, else read from
-// global memory); four partial sums per row keep four column loads in flight.
+// global memory); eight columns are read at a time and added to four partial sums.
+// Each thread has one 16-byte piece of w (ALN: every column starts on such a
+// boundary), else one value.
 constexpr int GN_MAX = 1024;
-template <typename S, bool C>
+template <typename S, bool C, bool ALN>
 __global__ void __launch_bounds__(256) k_gemv_n(int64_t len, int k, const S *V, int64_t ld,
                                                 const double *coef, S *w, bool sub) {
   __shared__ double cs[2 * GN_MAX];
@@ -965,44 +1004,58 @@ __global__ void __launch_bounds__(256) k_gemv_n(int64_t len, int k, const S *V, 
     for (int t = threadIdx.x; t < 2 * k; t += blockDim.x) cs[t] = coef[t];
   __syncthreads();
   const double *cf = staged ? cs : coef;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    double sr[4] = {0.0, 0.0, 0.0, 0.0}, si[4] = {0.0, 0.0, 0.0, 0.0};
-    int j = 0;
-    for (; j + 4 <= k; j += 4) {
+  constexpr int E = ALN ? 16 / (int)sizeof(S) : (C ? 2 : 1);
+  struct alignas(ALN ? 16 : sizeof(S)) Chunk { S v[E]; };
+  const int64_t values = C ? 2 * len : len, cols = C ? 2 * ld : ld;
+  // the piece at value index at, of cnt values
+  auto piece = [&](int64_t at, int cnt, auto load, auto store) {
+    double s[4][E];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const double cr = cf[2 * (j + u)], ci = cf[2 * (j + u) + 1];
-        if constexpr (C) {
-          const S *vj = V + (size_t)(j + u) * ld * 2;
-          const double vr = vj[2 * i], vi = vj[2 * i + 1];
-          sr[u] += cr * vr - ci * vi;
-          si[u] += cr * vi + ci * vr;
-        } else {
-          sr[u] += cr * (double)V[(size_t)(j + u) * ld + i];
-        }
-      }
-    }
-    for (; j < k; ++j) {
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int e = 0; e < E; ++e) s[u][e] = 0.0;
+    auto add = [&](const Chunk &v, int j, double (&t)[E]) {
       const double cr = cf[2 * j], ci = cf[2 * j + 1];
       if constexpr (C) {
-        const S *vj = V + (size_t)j * ld * 2;
-        const double vr = vj[2 * i], vi = vj[2 * i + 1];
-        sr[0] += cr * vr - ci * vi;
-        si[0] += cr * vi + ci * vr;
+#pragma unroll
+        for (int e = 0; e < E; e += 2) {
+          t[e] += cr * (double)v.v[e] - ci * (double)v.v[e + 1];
+          t[e + 1] += cr * (double)v.v[e + 1] + ci * (double)v.v[e];
+        }
       } else {
-        sr[0] += cr * (double)V[(size_t)j * ld + i];
+#pragma unroll
+        for (int e = 0; e < E; ++e) t[e] += cr * (double)v.v[e];
       }
+    };
+    int j = 0;
+    for (; j + 8 <= k; j += 8) {
+      Chunk v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = load(V + (size_t)(j + u) * cols + at, cnt);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) add(v[u], j + u, s[u & 3]);
     }
-    const double tr = (sr[0] + sr[1]) + (sr[2] + sr[3]);
-    const double ti = (si[0] + si[1]) + (si[2] + si[3]);
-    if constexpr (C) {
-      if (sub) { w[2 * i] = (S)((double)w[2 * i] - tr); w[2 * i + 1] = (S)((double)w[2 * i + 1] - ti); }
-      else { w[2 * i] = (S)tr; w[2 * i + 1] = (S)ti; }
-    } else {
-      w[i] = sub ? (S)((double)w[i] - tr) : (S)tr;
+    for (; j + 4 <= k; j += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) add(load(V + (size_t)(j + u) * cols + at, cnt), j + u, s[u]);
     }
-  }
+    for (; j < k; ++j) add(load(V + (size_t)j * cols + at, cnt), j, s[0]);
+    Chunk o = sub ? load(w + at, cnt) : Chunk{};
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const double t = (s[0][e] + s[1][e]) + (s[2][e] + s[3][e]);
+      o.v[e] = sub ? (S)((double)o.v[e] - t) : (S)t;
+    }
+    store(w + at, o, cnt);
+  };
+  const int64_t chunks = values / E;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < chunks; i += (int64_t)gridDim.x * blockDim.x)
+    piece(i * E, E, [](const S *p, int) { return *reinterpret_cast<const Chunk *>(p); },
+          [](S *p, const Chunk &c, int) { *reinterpret_cast<Chunk *>(p) = c; });
+  if (chunks * E < values && blockIdx.x == 0 && threadIdx.x == 0)
+    piece(chunks * E, (int)(values - chunks * E),
+          [](const S *p, int cnt) { Chunk c{}; for (int e = 0; e < cnt; ++e) c.v[e] = p[e]; return c; },
+          [](S *p, const Chunk &c, int cnt) { for (int e = 0; e < cnt; ++e) p[e] = c.v[e]; });
 }
 
 // Gaussian start vector from a counter-based hash (Box-Muller).
@@ -1354,49 +1407,61 @@ int launch_gemv_t(el_ctx *ctx, int dtype, int64_t len, int k, const void *V,
   const int gcap = std::max(1, (2 * sms + ngroups - 1) / ngroups);   // about two CTAs per SM in total
   if (gx > gcap) gx = gcap;
   dim3 grid(gx, ngroups);
+  const bool aln = (((uintptr_t)V | (uintptr_t)w | ((size_t)ld * dtype_size(dtype))) & 15) == 0;
   int rc = ensure_partials(ctx, (size_t)gx * k * 2);
   if (rc) return rc;
   switch (dtype) {
-    case EL_F32: k_gemv_t<float, false><<<grid, 256, 0, ctx->stream>>>(len, k, (const float *)V, ld, (const float *)w, ctx->d_partials); break;
-    case EL_F64: k_gemv_t<double, false><<<grid, 256, 0, ctx->stream>>>(len, k, (const double *)V, ld, (const double *)w, ctx->d_partials); break;
-    case EL_C64: k_gemv_t<float, true><<<grid, 256, 0, ctx->stream>>>(len, k, (const float *)V, ld, (const float *)w, ctx->d_partials); break;
-    case EL_C128: k_gemv_t<double, true><<<grid, 256, 0, ctx->stream>>>(len, k, (const double *)V, ld, (const double *)w, ctx->d_partials); break;
+#define EL_GEMVT(S, C)                                                                                            \
+  do {                                                                                                            \
+    if (aln) k_gemv_t<S, C, true><<<grid, 256, 0, ctx->stream>>>(len, k, (const S *)V, ld, (const S *)w, ctx->d_partials); \
+    else k_gemv_t<S, C, false><<<grid, 256, 0, ctx->stream>>>(len, k, (const S *)V, ld, (const S *)w, ctx->d_partials);    \
+  } while (0)
+    case EL_F32: EL_GEMVT(float, false); break;
+    case EL_F64: EL_GEMVT(double, false); break;
+    case EL_C64: EL_GEMVT(float, true); break;
+    case EL_C128: EL_GEMVT(double, true); break;
+#undef EL_GEMVT
     default: return fail(ctx, EL_EINVAL, "unknown dtype %d", dtype);
   }
   EL_LAUNCH_CHECK(ctx);
-  k_sum_partials<<<(2 * k + 255) / 256, 256, 0, ctx->stream>>>(gx, k, ctx->d_partials, dots_out);
+  k_sum_partials<<<(2 * k + 31) / 32, 256, 0, ctx->stream>>>(gx, k, ctx->d_partials, dots_out);
+  EL_LAUNCH_CHECK(ctx);
+  return EL_OK;
+}
+
+static int gemv_n(el_ctx *ctx, int dtype, int64_t len, int k, const void *V, int64_t ld, const double *coef,
+                  void *w, bool sub) {
+  if (k <= 0) return EL_OK;
+  const int es = dtype_size(dtype);
+  if (!es) return fail(ctx, EL_EINVAL, "unknown dtype %d", dtype);
+  // pieces where they still fill the GPU: a thread's columns are a chain of reads
+  const bool aln = (((uintptr_t)V | (uintptr_t)w | ((size_t)ld * es)) & 15) == 0 &&
+                   len * es / 16 >= (int64_t)sm_count(ctx) * 1024;
+  const int grid = grid_for(aln ? (len * es + 15) / 16 : len, 256);
+#define EL_GEMVN(S, C)                                                                                         \
+  do {                                                                                                         \
+    if (aln) k_gemv_n<S, C, true><<<grid, 256, 0, ctx->stream>>>(len, k, (const S *)V, ld, coef, (S *)w, sub); \
+    else k_gemv_n<S, C, false><<<grid, 256, 0, ctx->stream>>>(len, k, (const S *)V, ld, coef, (S *)w, sub);    \
+  } while (0)
+  switch (dtype) {
+    case EL_F32: EL_GEMVN(float, false); break;
+    case EL_F64: EL_GEMVN(double, false); break;
+    case EL_C64: EL_GEMVN(float, true); break;
+    default: EL_GEMVN(double, true); break;
+  }
+#undef EL_GEMVN
   EL_LAUNCH_CHECK(ctx);
   return EL_OK;
 }
 
 int launch_gemv_n_sub(el_ctx *ctx, int dtype, int64_t len, int k, const void *V,
                       int64_t ld, const double *coef, void *w) {
-  if (k <= 0) return EL_OK;
-  const int grid = grid_for(len, 256);
-  switch (dtype) {
-    case EL_F32: k_gemv_n<float, false><<<grid, 256, 0, ctx->stream>>>(len, k, (const float *)V, ld, coef, (float *)w, true); break;
-    case EL_F64: k_gemv_n<double, false><<<grid, 256, 0, ctx->stream>>>(len, k, (const double *)V, ld, coef, (double *)w, true); break;
-    case EL_C64: k_gemv_n<float, true><<<grid, 256, 0, ctx->stream>>>(len, k, (const float *)V, ld, coef, (float *)w, true); break;
-    case EL_C128: k_gemv_n<double, true><<<grid, 256, 0, ctx->stream>>>(len, k, (const double *)V, ld, coef, (double *)w, true); break;
-    default: return fail(ctx, EL_EINVAL, "unknown dtype %d", dtype);
-  }
-  EL_LAUNCH_CHECK(ctx);
-  return EL_OK;
+  return gemv_n(ctx, dtype, len, k, V, ld, coef, w, true);
 }
 
 int launch_gemv_n(el_ctx *ctx, int dtype, int64_t len, int k, const void *V,
                   int64_t ld, const double *coef_dev, void *out) {
-  if (k <= 0) return EL_OK;
-  const int grid = grid_for(len, 256);
-  switch (dtype) {
-    case EL_F32: k_gemv_n<float, false><<<grid, 256, 0, ctx->stream>>>(len, k, (const float *)V, ld, coef_dev, (float *)out, false); break;
-    case EL_F64: k_gemv_n<double, false><<<grid, 256, 0, ctx->stream>>>(len, k, (const double *)V, ld, coef_dev, (double *)out, false); break;
-    case EL_C64: k_gemv_n<float, true><<<grid, 256, 0, ctx->stream>>>(len, k, (const float *)V, ld, coef_dev, (float *)out, false); break;
-    case EL_C128: k_gemv_n<double, true><<<grid, 256, 0, ctx->stream>>>(len, k, (const double *)V, ld, coef_dev, (double *)out, false); break;
-    default: return fail(ctx, EL_EINVAL, "unknown dtype %d", dtype);
-  }
-  EL_LAUNCH_CHECK(ctx);
-  return EL_OK;
+  return gemv_n(ctx, dtype, len, k, V, ld, coef_dev, out, false);
 }
 
 int launch_fill_gauss(el_ctx *ctx, int dtype, int64_t len, uint64_t seed, void *out) {

@@ -322,35 +322,45 @@ extern "C" int el_lanczos_ground(el_ctx *ctx, el_ham *h, int dtype, const void *
     bool force_next = false;
     int j = 0;
     bool invariant = false;
-    int last_check = -1;
+    int last_check = -1, check_gap = 4;
     // Steps [j, queued) are on the stream: H v_j - beta v_{j-1} with its dot,
     // the update and the scaling of v_{j+1}, all scalars on the device
-    // (rec: alpha, |w|^2, -beta, -).  The host reads them together and goes
-    // through the steps in order; where one has to be reorthogonalised, the
-    // steps after it are queued again.
-    int queued = 0, read = 0;
+    // (rec: alpha, |w|^2, -beta, -).  The host reads them together, goes
+    // through the steps in order and queues the next ones before it looks at
+    // the Ritz values, which take it longer than the GPU takes for a few
+    // steps; where a step has to be reorthogonalised, the ones after it are
+    // queued again.
+    int queued = 0, read = 0, have = 0;      // scalars of steps [read, have) are on the host
+    auto queue = [&](int from, double bprev, int count) -> int {
+      for (int q = from; q < from + count; ++q) {
+        ApplyArgs A;
+        memset(&A, 0, sizeof A);
+        A.dtype = dtype; A.nvec = 1; A.x = Vj(q); A.z = q ? Vj(q - 1) : nullptr; A.y = Vj(q + 1);
+        A.a = 1.0; A.c = -bprev; A.c_dev = q > from ? rec + 4 * (q - 1) + 2 : nullptr; A.dots = d_sc; A.want_dots = 2;
+        int rq = el::launch_apply(ctx, h, A);
+        if (rq) return rq;
+        rq = el::launch_lanczos_update(ctx, dtype, dim, Vj(q), Vj(q + 1), d_sc, nullptr, rec + 4 * q);
+        if (rq) return rq;
+        rq = el::launch_scale(ctx, dtype, dim, rec + 4 * q + 1, 1, Vj(q + 1));
+        if (rq) return rq;
+      }
+      queued = from + count;
+      return EL_OK;
+    };
     for (j = 0; j < m; ++j) {
       if (el::cancelled(ctx)) return fail(ctx, EL_ECANCEL, "cancelled");
       const double bj = j ? be[j - 1] : 0.0;
       if (j == queued) {
-        const int nb = std::min(force_next || reorth == 2 ? 1 : steps_ahead(vb), m - j);
-        for (int q = j; q < j + nb; ++q) {
-          ApplyArgs A;
-          memset(&A, 0, sizeof A);
-          A.dtype = dtype; A.nvec = 1; A.x = Vj(q); A.z = q ? Vj(q - 1) : nullptr; A.y = Vj(q + 1);
-          A.a = 1.0; A.c = -bj; A.c_dev = q > j ? rec + 4 * (q - 1) + 2 : nullptr; A.dots = d_sc; A.want_dots = 2;
-          rc = el::launch_apply(ctx, h, A);
-          if (rc) return rc;
-          rc = el::launch_lanczos_update(ctx, dtype, dim, Vj(q), Vj(q + 1), d_sc, nullptr, rec + 4 * q);
-          if (rc) return rc;
-          rc = el::launch_scale(ctx, dtype, dim, rec + 4 * q + 1, 1, Vj(q + 1));
-          if (rc) return rc;
-        }
-        hr.resize(4 * (size_t)nb);
-        rc = sync_read(ctx, rec + 4 * j, 4 * nb, hr.data());
+        rc = queue(j, bj, std::min(force_next || reorth == 2 ? 1 : steps_ahead(vb), m - j));
         if (rc) return rc;
-        queued = j + nb;
+        have = j;
+      }
+      if (j == have) {
+        hr.resize(4 * (size_t)(queued - j));
+        rc = sync_read(ctx, rec + 4 * j, 4 * (queued - j), hr.data());
+        if (rc) return rc;
         read = j;
+        have = queued;
       }
       const double alpha = hr[4 * (j - read)];
       n2 = hr[4 * (j - read) + 1];
@@ -396,7 +406,7 @@ extern "C" int el_lanczos_ground(el_ctx *ctx, el_ham *h, int dtype, const void *
         rc = sync_read(ctx, d_sc + 8, 1, &n2);
         if (rc) return rc;
         bnext *= std::sqrt(std::max(n2, 0.0));
-        queued = j + 1;         // the steps after this one started from the old vector
+        queued = have = j + 1;  // the steps after this one started from the old vector
         if (reorth == 1) {
           for (int k = 0; k <= j; ++k) wnext[k] = eps;
           wnext[j + 1] = 1.0;
@@ -413,16 +423,24 @@ extern "C" int el_lanczos_ground(el_ctx *ctx, el_ham *h, int dtype, const void *
       const bool last = (j + 1 == m);
       const double scale = std::max(1.0, anorm);
       invariant = !(bnext > 1e-12 * scale);
-      // convergence check every few steps
-      if (mm >= nev && (invariant || last || mm - last_check >= 4)) {
+      // the next steps run while the host looks at the Ritz values
+      if (j + 1 == queued && !last && !invariant && !force_next && reorth != 2 && steps_ahead(vb) > 1) {
+        rc = queue(j + 1, bnext, std::min(steps_ahead(vb), m - j - 1));
+        if (rc) return rc;
+      }
+      // convergence check every few steps, less often far from convergence
+      if (mm >= nev && (invariant || last || mm - last_check >= check_gap)) {
         last_check = mm;
         bool ok = true;
+        double worst = 0.0;
         for (int q = 0; q < nev && q < mm; ++q) {
           theta[q] = el::tridiag_eig(al.data(), be.data(), mm, q);
           el::tridiag_vec(al.data(), be.data(), mm, theta[q], svec[q]);
           const double est = bnext * std::fabs(svec[q][mm - 1]);
           if (!(est <= 0.1 * tol * std::max(1.0, std::fabs(theta[q])))) ok = false;
+          worst = std::max(worst, est / (0.1 * tol * std::max(1.0, std::fabs(theta[q]))));
         }
+        check_gap = worst > 1e4 ? 16 : 4;
         if (ok || invariant || last) { j = mm; break; }
       }
       be.push_back(bnext);
