@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(NT) k_lanczos_batch(const BatchArgs A) {
 // ------------------------------------------------ one instance, whole GPU
 // Cooperative Lanczos for one instance that is too small to fill the GPU
 // with vectors but too slow on one SM: the rows are split over G CTAs (NT
-// rows each, one row per thread) and every CTA keeps its slice of the
+// rows each, one to four threads per row) and every CTA keeps its slice of the
 // Krylov basis in shared memory, so the full reorthogonalisation (classical
 // Gram-Schmidt, twice, every step) touches only shared memory; the
 // coefficients are summed across CTAs through small global arrays.  A step
@@ -773,6 +773,12 @@ __host__ __device__ inline size_t coop_slice_bytes(int m, int nt, int es) {
 }
 constexpr size_t COOP_WORK_BYTES = 2 * (6 * MAXIT + 8) * sizeof(double);
 
+// Threads per row of a CTA of nt rows: a row's flips and its Gram-Schmidt
+// update are split between them, and the columns of the projections have as
+// many threads (64 rows, 200 columns: one column each instead of three or
+// four in turn).
+__host__ __device__ constexpr int coop_tp(int nt) { return nt <= 128 ? 4 : nt <= 256 ? 2 : 1; }
+
 // Per-CTA partial sums of the ground-state occupations: x = sum_j y_j v_j on
 // this thread's row (v_j in the CTA's Krylov slice), out[k] = sum over the
 // CTA's rows of x^2 bit_k, out[n] = sum of x^2 (kept out of line: it runs
@@ -781,26 +787,29 @@ template <typename T, int NT>
 __device__ __noinline__ void coop_occupation_partials(const double *y, const T *Vs, int pitch, int steps,
                                                       bool valid, uint64_t code, int n, double *red,
                                                       double *out) {
+  constexpr int NTH = NT * coop_tp(NT);
   double x = 0.0;
-  if (valid)
+  if (valid && threadIdx.x < NT)
     for (int jj = 0; jj < steps; ++jj) x += y[jj] * (double)Vs[(size_t)jj * pitch + threadIdx.x];
   const double p2 = x * x;
   for (int k = 0; k < n; ++k) {
-    const double sk = block_sum<NT>(((code >> k) & 1ULL) ? p2 : 0.0, red);
+    const double sk = block_sum<NTH>(((code >> k) & 1ULL) ? p2 : 0.0, red);
     if (threadIdx.x == 0) out[k] = sk;
   }
-  const double tot = block_sum<NT>(p2, red);
+  const double tot = block_sum<NTH>(p2, red);
   if (threadIdx.x == 0) out[n] = tot;
 }
 
 template <typename T, int NT>
-__global__ void __launch_bounds__(NT) k_lanczos_coop(const CoopArgs G) {
+__global__ void __launch_bounds__(NT * coop_tp(NT), 1) k_lanczos_coop(const CoopArgs G) {
+  constexpr int TP = coop_tp(NT), NTH = NT * TP;
   extern __shared__ __align__(16) unsigned char coop_smem[];
   T *Vs = reinterpret_cast<T *>(coop_smem);           // [m + 1][NT + 1]
   constexpr int PITCH = NT + 1;
   __shared__ Inst I;
   __shared__ uint64_t fib[MAXN + 3];
-  __shared__ double red[NT / 32 > 0 ? NT / 32 : 1];
+  __shared__ double red[NTH / 32 > 0 ? NTH / 32 : 1];
+  __shared__ double psum[TP][NT];          // the parts' sums of a row
   __shared__ double al[MAXIT], be[MAXIT];
   __shared__ double cs[MAXIT + 2];
   __shared__ T wsm[NT];
@@ -820,8 +829,21 @@ __global__ void __launch_bounds__(NT) k_lanczos_coop(const CoopArgs G) {
   }
   __syncthreads();
   const int64_t dim = I.dim;
-  const int64_t row = (int64_t)blockIdx.x * NT + tid;
+  const int rt = tid % NT, part_ = tid / NT;   // row of the CTA, share of its work
+  const bool lead = part_ == 0;                // finishes and stores the row
+  const int64_t row = (int64_t)blockIdx.x * NT + rt;
   const bool valid = row < dim;
+  // the sum of the parts' values of each row, in every part
+  auto row_sum = [&](double v) -> double {
+    if constexpr (TP == 1) return v;
+    psum[part_][rt] = v;
+    __syncthreads();
+    double s = psum[0][rt];
+#pragma unroll
+    for (int q = 1; q < TP; ++q) s += psum[q][rt];
+    __syncthreads();
+    return s;
+  };
   const double *D = G.diag + I.off;
   T *vpub = reinterpret_cast<T *>(G.vpub);
   const int m = (int)min((int64_t)G.m, dim);
@@ -840,20 +862,20 @@ __global__ void __launch_bounds__(NT) k_lanczos_coop(const CoopArgs G) {
     grid_barrier(G, gen);
     const int lane = tid & 31, warp = tid >> 5;
     double *tt = G.tot + (size_t)slot * (MAXIT + 2);
-    for (int k = blockIdx.x + warp * G.nctas; k < nk; k += G.nctas * (NT / 32)) {
+    for (int k = blockIdx.x + warp * G.nctas; k < nk; k += G.nctas * (NTH / 32)) {
       double v = 0.0;
       for (int cc = lane; cc < G.nctas; cc += 32) v += __ldcg(part(slot, cc, k));
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
       if (lane == 0) tt[k] = v;
     }
     grid_barrier(G, gen);
-    for (int k = tid; k < nk; k += NT) cs[k] = __ldcg(&tt[k]);
+    for (int k = tid; k < nk; k += NTH) cs[k] = __ldcg(&tt[k]);
     slot ^= 1;
     __syncthreads();
   };
   // sum over CTAs of a block-reduced scalar
   auto grid_scalar = [&](double v) -> double {
-    v = block_sum<NT>(v, red);
+    v = block_sum<NTH>(v, red);
     if (tid == 0) *part(slot, blockIdx.x, 0) = v;
     reduce_all(1);
     return cs[0];
@@ -867,11 +889,11 @@ __global__ void __launch_bounds__(NT) k_lanczos_coop(const CoopArgs G) {
     const double u2 = (h2 >> 11) * (1.0 / 9007199254740992.0);
     x0 = (double)(T)(sqrt(-2.0 * log(u1)) * cospi(2.0 * u2));
   }
-  const double n0 = grid_scalar(x0 * x0);
+  const double n0 = grid_scalar(lead ? x0 * x0 : 0.0);
   {
     const T v = (T)(x0 / sqrt(n0));
-    Vs[tid] = valid ? v : (T)0;
-    if (valid) vpub[row] = v;
+    if (lead) Vs[rt] = valid ? v : (T)0;
+    if (lead && valid) vpub[row] = v;
   }
   grid_barrier(G, gen);
   int steps = 0;
@@ -885,53 +907,53 @@ __global__ void __launch_bounds__(NT) k_lanczos_coop(const CoopArgs G) {
     double w = 0.0;
     if (valid) {
       const uint64_t code = unrank_b(I, fib, row);
-      w = D[row] * (double)Vs[(size_t)j * PITCH + tid];
-      for (int k = 0; k < I.n; ++k) {
+      if (lead) w = D[row] * (double)Vs[(size_t)j * PITCH + rt];
+      for (int k = part_; k < I.n; k += TP) {
         const double amp = I.om[k];
         if (amp == 0.0) continue;
         const int64_t t = flip_b(I, fib, code, row, k);
         if (t >= 0) w += amp * (double)__ldcg(&vpub[t]);
       }
     }
+    w = row_sum(w);
     // classical Gram-Schmidt against v_0..v_j, G.passes times; alpha = sum
     // of the v_j coefficients.  The last pass also sums |w|^2 (slot j + 1).
     double alpha = 0.0, b2 = 0.0;
     for (int pass = 0; pass < G.passes; ++pass) {
       const int last_pass = (pass == G.passes - 1);
-      wsm[tid] = (T)w;
+      if (lead) wsm[rt] = (T)w;
       __syncthreads();
-      for (int k = tid; k <= j; k += NT) {
+      for (int k = tid; k <= j; k += NTH) {
         const T *vk = Vs + (size_t)k * PITCH;
-        double c0 = 0.0, c1 = 0.0;
-        int r = 0;
-        for (; r + 1 < NT; r += 2) {
-          c0 += (double)vk[r] * (double)wsm[r];
-          c1 += (double)vk[r + 1] * (double)wsm[r + 1];
-        }
-        for (; r < NT; ++r) c0 += (double)vk[r] * (double)wsm[r];
-        *part(slot, blockIdx.x, k) = c0 + c1;
+        double c[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+        for (int r = 0; r < NT; r += 4)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) c[q] += (double)vk[r + q] * (double)wsm[r + q];
+        *part(slot, blockIdx.x, k) = (c[0] + c[1]) + (c[2] + c[3]);
       }
       if (last_pass) {
-        const double ww = block_sum<NT>(valid ? w * w : 0.0, red);
+        const double ww = block_sum<NTH>(valid && lead ? w * w : 0.0, red);
         if (tid == 0) *part(slot, blockIdx.x, j + 1) = ww;
       }
       reduce_all(j + 1 + last_pass);
       alpha += cs[j];
       if (last_pass) {
+        // |c|^2 by all threads: one thread's sum over 200 terms is as long
+        // as the whole projection
         double cc2 = 0.0;
-        for (int k = 0; k <= j; ++k) cc2 += cs[k] * cs[k];
+        for (int k = tid; k <= j; k += NTH) cc2 += cs[k] * cs[k];
+        cc2 = block_sum<NTH>(cc2, red);
         b2 = cs[j + 1] - cc2;
       }
-      if (valid) {
-        double acc0 = w, acc1 = 0.0;
-        int k = 0;
-        for (; k + 1 <= j; k += 2) {
-          acc0 -= cs[k] * (double)Vs[(size_t)k * PITCH + tid];
-          acc1 -= cs[k + 1] * (double)Vs[(size_t)(k + 1) * PITCH + tid];
-        }
-        for (; k <= j; ++k) acc0 -= cs[k] * (double)Vs[(size_t)k * PITCH + tid];
-        w = (double)(T)(acc0 + acc1);
-      }
+      double sub[4] = {0.0, 0.0, 0.0, 0.0};
+      int k = part_;
+      for (; k + 3 * TP <= j; k += 4 * TP)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sub[q] += cs[k + q * TP] * (double)Vs[(size_t)(k + q * TP) * PITCH + rt];
+      for (; k <= j; k += TP) sub[0] += cs[k] * (double)Vs[(size_t)k * PITCH + rt];
+      const double proj = row_sum((sub[0] + sub[1]) + (sub[2] + sub[3]));
+      if (valid) w = (double)(T)(w - proj);
       __syncthreads();
     }
     bnext = sqrt(fmax(b2, 0.0));
@@ -999,8 +1021,8 @@ __global__ void __launch_bounds__(NT) k_lanczos_coop(const CoopArgs G) {
     if (s_done) break;
     // v_{j+1} = w / beta, into the shared slice and the published vector
     const T vn = (T)(w / bnext);
-    Vs[(size_t)(j + 1) * PITCH + tid] = valid ? vn : (T)0;
-    if (valid) vpub[row] = vn;
+    if (lead) Vs[(size_t)(j + 1) * PITCH + rt] = valid ? vn : (T)0;
+    if (lead && valid) vpub[row] = vn;
     grid_barrier(G, gen);
   }
   if (G.nat) {
@@ -1489,9 +1511,10 @@ int el_batch_run_coop(el_ctx *ctx, el_batch *b, int reorth_passes, int check_eve
 #undef EL_CPICK
     EL_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
     int per_sm = 0;
-    EL_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, P.nt, P.smem));
+    const int threads = P.nt * coop_tp(P.nt);
+    EL_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, P.smem));
     if (per_sm * sms < P.nctas) return fail(ctx, EL_EINVAL, "cooperative grid of %d CTAs is not co-resident", P.nctas);
-    EL_CUDA_TRY(ctx, cudaLaunchCooperativeKernel(fn, dim3(P.nctas), dim3(P.nt), kargs, P.smem, ctx->stream));
+    EL_CUDA_TRY(ctx, cudaLaunchCooperativeKernel(fn, dim3(P.nctas), dim3(threads), kargs, P.smem, ctx->stream));
     ctx->launches++;
   }
   // a barrier that timed out leaves the flag set
