@@ -84,21 +84,27 @@ __device__ __forceinline__ void rescale2(double &p, double &q) {
   }
 }
 
+// Power of two that brings numbers up to `scale` below 1.
+__device__ __forceinline__ double unit_scale(double scale) { return scalbn(1.0, -(ilogb(fmax(scale, 1e-300)) + 1)); }
+
 // Number of eigenvalues of T below x: the number of k in 1..m at which
 // chi_k(x) and chi_{k-1}(x) have the same sign (a zero counts as the sign
-// opposite to its predecessor).
-__device__ int sturm(const double *a, const double *b, int m, double x) {
+// opposite to its predecessor).  us: unit_scale of T's entries; with x - a and
+// b times it below 2 the pair can only grow or shrink so far in 8 steps, so it
+// is rescaled every 8th (the test in every step was two thirds of the chain).
+__device__ int sturm(const double *a, const double *b, int m, double x, double us) {
   int cnt = 0;
-  double pm = 1.0, p = x - a[0];
+  double pm = 1.0, p = (x - a[0]) * us;
   double sprev = 1.0;
   double sp = (p == 0.0) ? -sprev : p;
   if (sp > 0) ++cnt;
   sprev = sp;
   for (int i = 1; i < m; ++i) {
-    const double pn = fma(x - a[i], p, -(b[i - 1] * b[i - 1]) * pm);
+    const double bs = b[i - 1] * us;
+    const double pn = fma((x - a[i]) * us, p, -(bs * bs) * pm);
     pm = p;
     p = pn;
-    rescale2(p, pm);
+    if ((i & 7) == 0) rescale2(p, pm);
     const double s = (p == 0.0) ? -sprev : p;
     if ((s > 0) == (sprev > 0)) ++cnt;
     sprev = s;
@@ -107,11 +113,11 @@ __device__ int sturm(const double *a, const double *b, int m, double x) {
 }
 
 // k-th smallest eigenvalue by 32-way multisection within one warp.
-__device__ double warp_eig(const double *a, const double *b, int m, int k, double lo, double hi) {
+__device__ double warp_eig(const double *a, const double *b, int m, int k, double lo, double hi, double us) {
   const int lane = threadIdx.x & 31;
   for (int round = 0; round < 14; ++round) {
     const double x = lo + (hi - lo) * (lane + 1) / 33.0;
-    const int c = sturm(a, b, m, x);
+    const int c = sturm(a, b, m, x, us);
     const unsigned below = __ballot_sync(0xffffffffu, c > k);   // points above the eigenvalue
     const int first = below ? (__ffs(below) - 1) : 32;
     const double nlo = lo + (hi - lo) * first / 33.0;
@@ -123,51 +129,78 @@ __device__ double warp_eig(const double *a, const double *b, int m, int k, doubl
   return 0.5 * (lo + hi);
 }
 
-// Last component of the unit eigenvector of T for eigenvalue lam (inverse
-// iteration with a pivoted tridiagonal LU, one thread).
+// Last component of the unit eigenvector of T for eigenvalue lam: inverse
+// iteration with a pivoted tridiagonal LU by one warp (every lane calls it;
+// the factorisation and the solves run on lane 0, all element-wise work on
+// the 32 lanes).  work: 5 m doubles and m ints; the vector is left at
+// work + 4 m.
 __device__ double last_component(const double *a, const double *b, int m, double lam, double *work) {
-  if (m == 1) return 1.0;
+  const int lane = threadIdx.x & 31;
   double *d = work, *u1 = work + m, *u2 = work + 2 * m, *l = work + 3 * m, *x = work + 4 * m;
   int *piv = (int *)(work + 5 * m);
-  double scale = 0.0;
-  for (int i = 0; i < m; ++i) scale = fmax(scale, fabs(a[i]) + (i < m - 1 ? fabs(b[i]) : 0.0));
-  const double eps = 2.2e-16 * fmax(scale, 1e-300);
-  double cd = a[0] - lam, cu1 = b[0], cu2 = 0.0;
-  for (int i = 0; i < m - 1; ++i) {
-    const double sub = b[i], nd = a[i + 1] - lam, nu1 = (i + 1 < m - 1) ? b[i + 1] : 0.0;
-    if (fabs(cd) >= fabs(sub)) {
-      piv[i] = 0;
-      double dv = fabs(cd) < eps ? (cd < 0 ? -eps : eps) : cd;
-      const double f = sub / dv;
-      l[i] = f; d[i] = dv; u1[i] = cu1; u2[i] = cu2;
-      cd = nd - f * cu1; cu1 = nu1 - f * cu2; cu2 = 0.0;
-    } else {
-      piv[i] = 1;
-      const double f = cd / sub;
-      l[i] = f; d[i] = sub; u1[i] = nd; u2[i] = nu1;
-      cd = cu1 - f * nd; cu1 = cu2 - f * nu1; cu2 = 0.0;
-    }
+  if (m == 1) {
+    if (lane == 0) x[0] = 1.0;
+    __syncwarp();
+    return 1.0;
   }
-  d[m - 1] = fabs(cd) < eps ? (cd < 0 ? -eps : eps) : cd;
-  for (int i = 0; i < m; ++i) d[i] = 1.0 / d[i];            // reciprocal pivots
-  for (int i = 0; i < m; ++i) x[i] = 1.0 + 0.01 * sin(1.0 + i);
-  for (int it = 0; it < 3; ++it) {
+  double scale = 0.0;
+  for (int i = lane; i < m; i += 32) {
+    scale = fmax(scale, fabs(a[i]) + (i < m - 1 ? fabs(b[i]) : 0.0));
+    x[i] = 1.0 + 0.01 * sin(1.0 + i);
+  }
+  for (int o = 16; o > 0; o >>= 1) scale = fmax(scale, __shfl_xor_sync(0xffffffffu, scale, o));
+  const double eps = 2.2e-16 * fmax(scale, 1e-300);
+  if (lane == 0) {
+    double cd = a[0] - lam, cu1 = b[0], cu2 = 0.0;
     for (int i = 0; i < m - 1; ++i) {
-      if (piv[i]) { const double t = x[i]; x[i] = x[i + 1]; x[i + 1] = t; }
-      x[i + 1] -= l[i] * x[i];
+      const double sub = b[i], nd = a[i + 1] - lam, nu1 = (i + 1 < m - 1) ? b[i + 1] : 0.0;
+      if (fabs(cd) >= fabs(sub)) {
+        piv[i] = 0;
+        double dv = fabs(cd) < eps ? (cd < 0 ? -eps : eps) : cd;
+        const double f = sub / dv;
+        l[i] = f; d[i] = dv; u1[i] = cu1; u2[i] = cu2;
+        cd = nd - f * cu1; cu1 = nu1 - f * cu2; cu2 = 0.0;
+      } else {
+        piv[i] = 1;
+        const double f = cd / sub;
+        l[i] = f; d[i] = sub; u1[i] = nd; u2[i] = nu1;
+        cd = cu1 - f * nd; cu1 = cu2 - f * nu1; cu2 = 0.0;
+      }
     }
-    for (int i = m - 1; i >= 0; --i) {
-      double s = x[i];
-      if (i + 1 < m) s -= u1[i] * x[i + 1];
-      if (i + 2 < m) s -= u2[i] * x[i + 2];
-      x[i] = s * d[i];
+    d[m - 1] = fabs(cd) < eps ? (cd < 0 ? -eps : eps) : cd;
+  }
+  __syncwarp();
+  for (int i = lane; i < m; i += 32) d[i] = 1.0 / d[i];            // reciprocal pivots
+  __syncwarp();
+  for (int it = 0; it < 3; ++it) {
+    if (lane == 0) {
+      double xi = x[0];
+      for (int i = 0; i < m - 1; ++i) {
+        double xn = x[i + 1];
+        if (piv[i]) { const double t = xi; xi = xn; xn = t; }
+        x[i] = xi;
+        xi = xn - l[i] * xi;
+      }
+      x[m - 1] = xi;
+      double x1 = 0.0, x2 = 0.0;       // x[i + 1], x[i + 2]
+      for (int i = m - 1; i >= 0; --i) {
+        double s = x[i];
+        if (i + 1 < m) s -= u1[i] * x1;
+        if (i + 2 < m) s -= u2[i] * x2;
+        x2 = x1;
+        x1 = s * d[i];
+        x[i] = x1;
+      }
     }
+    __syncwarp();
     double nrm = 0.0;
-    for (int i = 0; i < m; ++i) nrm += x[i] * x[i];
+    for (int i = lane; i < m; i += 32) nrm += x[i] * x[i];
+    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
     nrm = sqrt(nrm);
-    if (!(nrm > 0) || !isfinite(nrm)) return 1.0;
+    if (!(nrm > 0) || !isfinite(nrm)) return 1.0;      // the same in every lane
     const double inv = 1.0 / nrm;
-    for (int i = 0; i < m; ++i) x[i] *= inv;
+    for (int i = lane; i < m; i += 32) x[i] *= inv;
+    __syncwarp();
   }
   return fabs(x[m - 1]);
 }
@@ -619,20 +652,22 @@ __global__ void __launch_bounds__(NT) k_lanczos_batch(const BatchArgs A) {
         glo -= 1e-9 * scale;
         ghi += 1e-9 * scale;
         const int ne = mm >= 2 ? 2 : 1;
+        const double us = unit_scale(2.0 * scale);
         double worst = 0.0;
         for (int q = 0; q < ne; ++q) {
           double lo = glo, hi = ghi;
           if (s_have) {
             hi = fmin(ghi, s_pth[q] + 1e-12 * scale);
             const double cand = hi - fmax(16.0 * s_pdth[q], 1e-10 * scale);
-            if (cand > glo && sturm(al, be, mm, cand) <= q) lo = cand;
+            if (cand > glo && sturm(al, be, mm, cand, us) <= q) lo = cand;
           }
-          const double th = warp_eig(al, be, mm, q, lo, hi);
+          const double th = warp_eig(al, be, mm, q, lo, hi, us);
+          const double tail = last_component(al, be, mm, th, work + 2 * MAXIT);
           if (tid == 0) {
             s_pdth[q] = s_have ? fmax(s_pth[q] - th, 0.0) : fabs(ghi - glo);
             s_pth[q] = th;
             s_th[q] = th;
-            s_res[q] = bnext * last_component(al, be, mm, th, work + 2 * MAXIT);
+            s_res[q] = bnext * tail;
             worst = fmax(worst, s_res[q] / (A.tol * fmax(1.0, fabs(th))));
           }
           __syncwarp();
@@ -673,10 +708,7 @@ __global__ void __launch_bounds__(NT) k_lanczos_batch(const BatchArgs A) {
       // (y: unit eigenvector of T for theta_0, by inverse iteration):
       // <n_k> = sum_r x_r^2 bit_k(r) / sum_r x_r^2, fixed-order block sums
       __syncthreads();
-      if (tid == 0) {
-        if (steps == 1) work[2 * MAXIT + 4] = 1.0;   // a one-vector Krylov space
-        else last_component(al, be, steps, s_th[0], work + 2 * MAXIT);
-      }
+      if (tid < 32) last_component(al, be, steps, s_th[0], work + 2 * MAXIT);
       __syncthreads();
       const double *y = work + 2 * MAXIT + 4 * steps;
       // lane l of each warp owns bit positions l and l + 32: the warp's rows
@@ -847,7 +879,7 @@ __global__ void __launch_bounds__(NT * coop_tp(NT), 1) k_lanczos_coop(const Coop
   const double *D = G.diag + I.off;
   T *vpub = reinterpret_cast<T *>(G.vpub);
   const int m = (int)min((int64_t)G.m, dim);
-  // inverse-iteration buffers of lanes 0 and 1 follow the slice in dynamic memory
+  // inverse-iteration buffers of the two Ritz pairs follow the slice in dynamic memory
   double *work = reinterpret_cast<double *>(coop_smem + coop_slice_bytes(m, NT, (int)sizeof(T)));
   unsigned gen = 0;
   int slot = 0;
@@ -968,54 +1000,57 @@ __global__ void __launch_bounds__(NT * coop_tp(NT), 1) k_lanczos_coop(const Coop
     // tridiagonal grows, so the previous value bounds it from above; a
     // Sturm count confirms a narrow lower bound below it (else the
     // Gershgorin bound is used), which saves most multisection rounds.  The
-    // two residual estimates (inverse iteration) run on lanes 0 and 1.
+    // two pairs (multisection and inverse iteration) run on two warps.
     const bool check = invariant || (j + 1 == m) || (steps >= next_check);
-    if (check && tid < 32) {
-      const int mm = steps;
-      double glo = 1e300, ghi = -1e300;
-      for (int i = 0; i < mm; ++i) {
-        const double rr = (i > 0 ? fabs(be[i - 1]) : 0.0) + (i + 1 < mm ? fabs(be[i]) : 0.0);
-        glo = fmin(glo, al[i] - rr);
-        ghi = fmax(ghi, al[i] + rr);
-      }
-      const double scale = fmax(1.0, fmax(fabs(glo), fabs(ghi)));
-      glo -= 1e-9 * scale;
-      ghi += 1e-9 * scale;
-      const int ne = mm >= 2 ? 2 : 1;
-      double th[2] = {0.0, 0.0};
-      for (int q = 0; q < ne; ++q) {
+    if (check && tid < 64) {
+      const int mm = steps, q = tid >> 5, ne = mm >= 2 ? 2 : 1;
+      if (q < ne) {
+        const int lane = tid & 31;
+        double glo = 1e300, ghi = -1e300;
+        for (int i = lane; i < mm; i += 32) {
+          const double rr = (i > 0 ? fabs(be[i - 1]) : 0.0) + (i + 1 < mm ? fabs(be[i]) : 0.0);
+          glo = fmin(glo, al[i] - rr);
+          ghi = fmax(ghi, al[i] + rr);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+          glo = fmin(glo, __shfl_xor_sync(0xffffffffu, glo, o));
+          ghi = fmax(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
+        }
+        const double scale = fmax(1.0, fmax(fabs(glo), fabs(ghi)));
+        glo -= 1e-9 * scale;
+        ghi += 1e-9 * scale;
+        const double us = unit_scale(2.0 * scale);
         double lo = glo, hi = ghi;
         if (have_prev) {
           hi = fmin(ghi, prev_th[q] + 1e-12 * scale);
           const double d = fmax(16.0 * prev_dth[q], 1e-10 * scale);
           const double cand = hi - d;
-          if (cand > glo && sturm(al, be, mm, cand) <= q) lo = cand;
+          if (cand > glo && sturm(al, be, mm, cand, us) <= q) lo = cand;
         }
-        th[q] = warp_eig(al, be, mm, q, lo, hi);
-      }
-      if (tid < ne) {
-        const double r = bnext * last_component(al, be, mm, th[tid], work + (size_t)tid * (6 * MAXIT + 8));
-        s_res[tid] = r;
-        s_th[tid] = th[tid];
-      }
-      __syncwarp();
-      if (tid == 0) {
-        bool ok = (ne == 2);
-        double worst = 0.0;
-        for (int q = 0; q < ne; ++q) {
-          const double lim = G.tol * fmax(1.0, fabs(s_th[q]));
-          ok = ok && (s_res[q] <= lim);
-          worst = fmax(worst, s_res[q] / lim);
+        const double th = warp_eig(al, be, mm, q, lo, hi, us);
+        const double tail = last_component(al, be, mm, th, work + (size_t)q * (6 * MAXIT + 8));
+        if (lane == 0) {
+          s_res[q] = bnext * tail;
+          s_th[q] = th;
+          prev_dth[q] = have_prev ? fmax(prev_th[q] - th, 0.0) : fabs(ghi - glo);
+          prev_th[q] = th;
         }
-        s_done = (ok || invariant || j + 1 == m) ? 1 : 0;
-        // far from converged: look again later
-        s_next = mm + (worst > 1e3 ? 4 : 1) * G.check_every;
       }
-      if (tid < ne) {
-        prev_dth[tid] = have_prev ? fmax(prev_th[tid] - th[tid], 0.0) : fabs(ghi - glo);
-        prev_th[tid] = th[tid];
+    }
+    __syncthreads();
+    if (check && tid == 0) {
+      const int ne = steps >= 2 ? 2 : 1;
+      bool ok = (ne == 2);
+      double worst = 0.0;
+      for (int q = 0; q < ne; ++q) {
+        const double lim = G.tol * fmax(1.0, fabs(s_th[q]));
+        ok = ok && (s_res[q] <= lim);
+        worst = fmax(worst, s_res[q] / lim);
       }
-      if (tid == 0) have_prev = 1;
+      s_done = (ok || invariant || j + 1 == m) ? 1 : 0;
+      // far from converged: look again later
+      s_next = steps + (worst > 1e3 ? 4 : 1) * G.check_every;
+      have_prev = 1;
     }
     __syncthreads();
     if (s_done) break;
@@ -1030,10 +1065,7 @@ __global__ void __launch_bounds__(NT * coop_tp(NT), 1) k_lanczos_coop(const Coop
     // kernel): every CTA forms y from the same alpha/beta, its rows of x from
     // its Krylov slice, and per-site partial sums that reduce_all adds up
     __syncthreads();
-    if (tid == 0) {
-      if (steps <= 1) work[4] = 1.0;
-      else last_component(al, be, steps, s_th[0], work);
-    }
+    if (tid < 32) last_component(al, be, steps <= 1 ? 1 : steps, s_th[0], work);
     __syncthreads();
     coop_occupation_partials<T, NT>(work + 4 * (steps <= 1 ? 1 : steps), Vs, PITCH, steps, valid,
                                     valid ? unrank_b(I, fib, row) : 0, I.n, red,
