@@ -16,7 +16,7 @@
 // from the step's checkpoint, another 1827 of 7186 phases), a step's last
 // reverse phase also writes lambda and the next step's u_M, and each thread
 // adds up its gradient dots over a step, one block sum per step.  20-site
-// ring, 200 steps, complex64: 22.8 -> 10.7 ms (14.9 with the row values read from memory in each phase).  Four lanes share a row (its
+// ring, 200 steps, complex64: 22.8 -> 11.0 ms (14.9 with the row values read from memory in each phase).  Four lanes share a row (its
 // flips split between them) as in k_adjoint_step, and keep its flip targets
 // in registers across all sweeps; every step's Chebyshev plan (a, b, M, c_m)
 // is computed on the host first and read from device arrays.  Gradient dots
@@ -44,6 +44,7 @@ struct CoopAdj {
   const double *pc;        // [K][Mmax + 1][2] coefficients c_m
   const double *om, *dl;   // [K] Omega_k and -Delta_k
   const S *diagV;          // the V part of the diagonal
+  const double *diag64;
   S ahalf[EL_MAX_SITES];   // a_i / 2 per bit position
   S bsh[EL_MAX_SITES];     // b_i per bit position
   S *ckp;                  // [K + 1][dim] complex checkpoints
@@ -227,7 +228,8 @@ __device__ __forceinline__ void sweep(const CoopAdj<S> &P, S om, S dl, const Swe
 // u_{m+1}, u_{m+2}, lambda, its diagonal) stay in registers of the row's first
 // lane, a step's coefficients come through shared memory, and the stored
 // term of the next phase is read before the barrier.  What a phase waits for
-// after its barrier is one round of flip partners.
+// after its barrier is one round of flip partners.  The row's own values are
+// FP64 also for FP32 vectors: only what is published is rounded.
 constexpr int MAXC = 256;   // terms of a step held in shared memory
 
 template <typename S>
@@ -255,41 +257,41 @@ __device__ __forceinline__ void gather_flips(const RowCache<S> &rc, const S *x, 
 template <typename S>
 __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, double *red, unsigned &gen) {
   typedef typename VecT<S, true>::type V2;
-  __shared__ S cbuf[2][2 * MAXC];
+  __shared__ double cbuf[2][2 * MAXC];
   __shared__ double s_ov[2];
   const size_t vs = (size_t)P.B.dim * 2;
   const bool mine = rc.active && (threadIdx.x & (CL - 1)) == 0;   // this thread finishes the row
   const int64_t r = rc.r;
   auto sync = [&]() { coop_sync(P.bar, P.err, P.nctas, P.poll_limit, gen); };
   auto at = [&](const S *p) { return reinterpret_cast<const V2 *>(p)[r]; };
-  auto put = [&](S *p, S re, S im) { V2 v; v.x = re; v.y = im; reinterpret_cast<V2 *>(p)[r] = v; };
+  auto put = [&](S *p, double re, double im) { V2 v; v.x = (S)re; v.y = (S)im; reinterpret_cast<V2 *>(p)[r] = v; };
   // coefficients of step k into buffer k & 1 (read after the next barrier)
   auto fetch = [&](int k) {
     if (k < 0 || k >= P.K) return;
     const double *c = P.pc + (size_t)k * (P.Mmax + 1) * 2;
-    for (int q = threadIdx.x; q < 2 * (P.pm[k] + 1); q += CNT) cbuf[k & 1][q] = (S)c[q];
+    for (int q = threadIdx.x; q < 2 * (P.pm[k] + 1); q += CNT) cbuf[k & 1][q] = c[q];
   };
-  const S diag = P.diagV[r];
+  const double diag = P.diag64[r];
   V2 x0 = at(P.ckp);
-  S xr = x0.x, xi = x0.y;       // own value of the vector the next sweep gathers
+  double xr = x0.x, xi = x0.y;       // own value of the vector the next sweep gathers
   fetch(0);
   __syncthreads();
   // ---- forward
   for (int k = 0; k < P.K; ++k) {
-    const S a = (S)P.pa[k], b = (S)P.pb[k], om = (S)P.om[k];
-    const S d = diag + (S)P.dl[k] * rc.nb;
+    const double a = P.pa[k], b = P.pb[k], om = P.om[k];
+    const double d = diag + P.dl[k] * (double)rc.nb;
     const int M = P.pm[k];
-    const S *c = cbuf[k & 1];
+    const double *c = cbuf[k & 1];
     S *term = P.term + (size_t)k * (P.Mmax + 1) * vs;
     S *out = P.ckp + (size_t)(k + 1) * vs;
     const S *x = P.ckp + (size_t)k * vs;
-    S zr = S(0), zi = S(0);
-    S accr = c[0] * xr - c[1] * xi, acci = c[0] * xi + c[1] * xr;
+    double zr = 0.0, zi = 0.0;
+    double accr = c[0] * xr - c[1] * xi, acci = c[0] * xi + c[1] * xr;
     for (int m = 1; m <= M; ++m) {
       S re, im;
       gather_flips<S>(rc, x, re, im);
-      const S al = (m == 1 ? S(1) : S(2)) / a, be = (m == 1 ? -b : S(-2) * b) / a;
-      const S yr = al * (d * xr + om * re) + be * xr - zr, yi = al * (d * xi + om * im) + be * xi - zi;
+      const double al = (m == 1 ? 1.0 : 2.0) / a, be = (m == 1 ? -b : -2.0 * b) / a;
+      const double yr = al * (d * xr + om * re) + be * xr - zr, yi = al * (d * xi + om * im) + be * xi - zi;
       accr += c[2 * m] * yr - c[2 * m + 1] * yi;
       acci += c[2 * m] * yi + c[2 * m + 1] * yr;
       zr = xr; zi = xi;
@@ -307,7 +309,7 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
     }
   }
   // ---- objective, lambda_K and u_M of the last step
-  S lr = S(0), li = S(0);
+  double lr = 0.0, li = 0.0;
   {
     double fa = 0.0, fb = 0.0;
     if (mine) {
@@ -327,13 +329,13 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
     if (blockIdx.x == 0 && threadIdx.x == 0) { P.fout[0] = s_ov[0]; P.fout[1] = s_ov[1]; }
     if (P.target) {   // lambda = <target, psi> target
       const V2 t = at(P.target);
-      lr = (S)s_ov[0] * t.x - (S)s_ov[1] * t.y;
-      li = (S)s_ov[0] * t.y + (S)s_ov[1] * t.x;
+      lr = s_ov[0] * t.x - s_ov[1] * t.y;
+      li = s_ov[0] * t.y + s_ov[1] * t.x;
     } else {          // lambda = O psi
-      lr = (S)P.obs[r] * xr;
-      li = (S)P.obs[r] * xi;
+      lr = P.obs[r] * xr;
+      li = P.obs[r] * xi;
     }
-    const S *c = cbuf[(P.K - 1) & 1];
+    const double *c = cbuf[(P.K - 1) & 1];
     const int M = P.pm[P.K - 1];
     xr = c[2 * M] * lr + c[2 * M + 1] * li;       // conj(c_M) lambda
     xi = c[2 * M] * li - c[2 * M + 1] * lr;
@@ -344,12 +346,12 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
   // ---- backward
   int us = 0;
   for (int k = P.K - 1; k >= 0; --k) {
-    const S a = (S)P.pa[k], b = (S)P.pb[k], om = (S)P.om[k];
-    const S d = diag + (S)P.dl[k] * rc.nb;
+    const double a = P.pa[k], b = P.pb[k], om = P.om[k];
+    const double d = diag + P.dl[k] * (double)rc.nb;
     const int M = P.pm[k], Mn = k > 0 ? P.pm[k - 1] : 0;
-    const S *c = cbuf[k & 1], *cn = cbuf[(k & 1) ^ 1];
+    const double *c = cbuf[k & 1], *cn = cbuf[(k & 1) ^ 1];
     const S *term = P.term + (size_t)k * (P.Mmax + 1) * vs;
-    S zr = S(0), zi = S(0);
+    double zr = 0.0, zi = 0.0;
     double gO = 0.0, gD = 0.0;
     if (M == 1 && k + 1 < P.K) {   // one phase: the next step's coefficients are needed in it
       fetch(k - 1);
@@ -359,10 +361,10 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
     for (int m = M - 1; m >= 0; --m) {
       S re, im;
       gather_flips<S>(rc, P.U + (size_t)us * vs, re, im);
-      const S al = (m == 0 ? S(1) : S(2)) / a, be = (m == 0 ? -b : S(-2) * b) / a;
+      const double al = (m == 0 ? 1.0 : 2.0) / a, be = (m == 0 ? -b : -2.0 * b) / a;
       // conj(c_m) lambda + (s/a)(H - b) u_{m+1} - u_{m+2}
-      const S yr = al * (d * xr + om * re) + be * xr - zr + (c[2 * m] * lr + c[2 * m + 1] * li);
-      const S yi = al * (d * xi + om * im) + be * xi - zi + (c[2 * m] * li - c[2 * m + 1] * lr);
+      const double yr = al * (d * xr + om * re) + be * xr - zr + (c[2 * m] * lr + c[2 * m + 1] * li);
+      const double yi = al * (d * xi + om * im) + be * xi - zi + (c[2 * m] * li - c[2 * m + 1] * lr);
       if (mine) {
         const double w = (m == 0) ? 1.0 : 2.0, tr = t.x, ti = t.y;
         gO += w * ((double)re * tr + (double)im * ti);                       // Re(conj(G_O u) t)
@@ -592,6 +594,7 @@ int adjoint_coop(el_ctx *ctx, el_ham *h, int K, const std::vector<ChebPlan> &pla
   P.pa = d_pa; P.pb = d_pb; P.pm = d_pm; P.pc = d_pc; P.om = d_om; P.dl = d_dl;
   if (std::is_same<S, float>::value) { int rc = el::ham_diag32(ctx, h); if (rc) return rc; }
   P.diagV = std::is_same<S, float>::value ? (const S *)(void *)h->d_diagV32 : (const S *)(void *)h->d_diagV64;
+  P.diag64 = h->d_diagV64;
   for (int q = 0; q < n; ++q) {
     P.ahalf[q] = (S)(0.5 * ash[n - 1 - q]);
     P.bsh[q] = (S)bsh[n - 1 - q];
