@@ -803,7 +803,7 @@ def native_ramp31(h, args):
     # t_{m-1} read and t_m written, accumulator read and written, diagonal read
     nterms = int(solve32.terms[0])
     rl = roofline(basis.dim * (3 * 8 + 2 * 8 + 4) * nterms, el / steps,
-                  kernel="k_apply_chain_tile (Chebyshev terms; whole solve: %d terms)" % nterms)
+                  kernel="k_chain_block (Chebyshev terms; whole solve: %d terms)" % nterms)
     rl["note"] = "state 28 MB: the recurrence vectors are largely L2-resident"
     line.update({
         "roofline": rl,

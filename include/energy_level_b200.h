@@ -143,7 +143,7 @@ int el_ham_set_loss(el_ctx *ctx, el_ham *ham, const double *gamma);
  * NULL (zero).  Targets outside a restricted basis are dropped, as for the
  * sigma^x channels.  A complex J or A makes H complex (complex vector dtypes
  * only).  n_pairs = 0 removes all exchange channels.  With exchange channels
- * every product runs the generic row kernel and KPM the generic recurrence.
+ * every product runs the hop or the generic kernel and KPM the generic recurrence.
  * Replaces the I2/I3 channels of channels.py:119-131 channel_spec. */
 int el_ham_set_exchange(el_ctx *ctx, el_ham *ham, int n_pairs, const int32_t *pi,
                         const int32_t *pj, const double *J_re, const double *J_im,
