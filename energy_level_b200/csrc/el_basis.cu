@@ -153,22 +153,22 @@ int build_tables(el_ctx *ctx, el_basis *b, int charge, int64_t max_states) {
 
 int upload_tables(el_ctx *ctx, el_basis *b) {
   const size_t npre = b->h_pre_off.size();
-  EL_CUDA_TRY(ctx, cudaMalloc(&b->d_pre_off, npre * sizeof(int64_t)));
-  EL_CUDA_TRY(ctx, cudaMalloc(&b->d_pre_cls, npre * sizeof(int32_t)));
-  EL_CUDA_TRY(ctx, cudaMalloc(&b->d_suf_rank, b->h_suf_rank.size() * sizeof(int32_t)));
-  EL_CUDA_TRY(ctx, el::copy(ctx, b->d_pre_off, b->h_pre_off.data(), npre * sizeof(int64_t), cudaMemcpyHostToDevice));
-  EL_CUDA_TRY(ctx, el::copy(ctx, b->d_pre_cls, b->h_pre_cls.data(), npre * sizeof(int32_t), cudaMemcpyHostToDevice));
-  EL_CUDA_TRY(ctx, el::copy(ctx, b->d_suf_rank, b->h_suf_rank.data(), b->h_suf_rank.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-  if (b->dim < ((int64_t)1 << 31)) {
-    std::vector<int2> pack(npre);
-    for (size_t p = 0; p < npre; ++p) {
-      const bool in = b->h_pre_off[p] >= 0;
-      pack[p].x = in ? (int)b->h_pre_off[p] : -1;
-      pack[p].y = in ? b->h_pre_cls[p] : 0;
-    }
-    EL_CUDA_TRY(ctx, cudaMalloc(&b->d_pre_pack, npre * sizeof(int2)));
-    EL_CUDA_TRY(ctx, el::copy(ctx, b->d_pre_pack, pack.data(), npre * sizeof(int2), cudaMemcpyHostToDevice));
+  // offsets, (offset, class) pairs and classes of the prefixes: one allocation, one upload
+  std::vector<char> tab(npre * 20);
+  int2 *const pack = reinterpret_cast<int2 *>(tab.data() + npre * 8);
+  memcpy(tab.data(), b->h_pre_off.data(), npre * 8);
+  memcpy(tab.data() + npre * 16, b->h_pre_cls.data(), npre * 4);
+  for (size_t p = 0; p < npre; ++p) {
+    const bool in = b->h_pre_off[p] >= 0;
+    pack[p].x = in ? (int)b->h_pre_off[p] : -1;      // used below 2^31 rows only
+    pack[p].y = in ? b->h_pre_cls[p] : 0;
   }
+  EL_CUDA_TRY(ctx, cudaMalloc(&b->d_pre_off, tab.size()));
+  b->d_pre_pack = reinterpret_cast<int2 *>((char *)b->d_pre_off + npre * 8);
+  b->d_pre_cls = reinterpret_cast<int32_t *>((char *)b->d_pre_off + npre * 16);
+  EL_CUDA_TRY(ctx, cudaMalloc(&b->d_suf_rank, b->h_suf_rank.size() * sizeof(int32_t)));
+  EL_CUDA_TRY(ctx, el::copy(ctx, b->d_pre_off, tab.data(), tab.size(), cudaMemcpyHostToDevice));
+  EL_CUDA_TRY(ctx, el::copy(ctx, b->d_suf_rank, b->h_suf_rank.data(), b->h_suf_rank.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
   // groups for the code expansion
   std::vector<uint64_t> gp;
   std::vector<int64_t> go;
@@ -329,8 +329,6 @@ int el_basis_destroy(el_basis *b) {
   if (!b) return EL_OK;
   cudaSetDevice(b->device);
   if (b->d_pre_off) cudaFree(b->d_pre_off);
-  if (b->d_pre_cls) cudaFree(b->d_pre_cls);
-  if (b->d_pre_pack) cudaFree(b->d_pre_pack);
   if (b->d_suf_rank) cudaFree(b->d_suf_rank);
   if (b->d_codes) cudaFree(b->d_codes);
   delete b;

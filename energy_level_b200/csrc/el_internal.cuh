@@ -66,6 +66,7 @@ struct el_basis {
   int64_t *d_pre_off = nullptr;
   int32_t *d_pre_cls = nullptr;
   int2 *d_pre_pack = nullptr;       // [2^P] (offset, class) in 32 bits, bases below 2^31 rows
+                                    // (d_pre_cls and d_pre_pack lie in d_pre_off's allocation)
   int32_t *d_suf_rank = nullptr;
   uint64_t *d_codes = nullptr;      // [dim] (TABLE layout only)
   int device = 0;
