@@ -17,9 +17,10 @@
 //     dF/dtheta_k = 2 sum_{m>=1} s_m Re <G_theta u_m, t_{m-1}> / a_k,
 // with G_Omega = sum a_i sigma^x_i / 2 and G_Delta = -sum b_i n_i.  a_k, b_k
 // are held fixed (the map depends on them only at the truncation level).
-// The forward pass keeps one state per step; the backward pass recomputes the
-// Chebyshev terms t_0..t_{M-1} of one step at a time from that checkpoint
-// (the recurrence is recomputed, never stored across steps).
+// The forward pass keeps one state per step and, in the cooperative gradient
+// while they fit STORE_MAX bytes, every step's Chebyshev terms; otherwise the
+// backward pass recomputes the terms t_0..t_{M-1} of one step at a time from
+// that checkpoint.
 #include "el_internal.cuh"
 
 #include <algorithm>

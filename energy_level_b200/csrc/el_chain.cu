@@ -1,21 +1,21 @@
 // Fused H-apply on nearest-neighbour chain and ring blockade sectors.
 //
-// A chain of n sites splits by code bit into L low, 4 middle and the
-// remaining high bits.  Rows that share the bits >= L + 4 (a tile) are
-// contiguous and ordered like the (L + 4)-site chain: 8 sub-blocks, one per
-// middle code 0000 0001 0010 0100 0101 1000 1001 1010 in this order, of
-// F(L+2) rows each (F(L+1) where middle bit 0 is set, because low bit L-1 is
-// then clear); a tile whose high bit L + 4 is set has the first five only.
-// A CTA takes one tile at a time and a thread one low code i and one
-// 16-byte chunk of the row (all vectors of a row are adjacent), for all
-// sub-blocks at once:
+// A chain of n sites splits by code bit into L low, 3 middle and the
+// remaining high bits.  Rows that share the bits >= L + 3 (a tile) are
+// contiguous and ordered like the (L + 3)-site chain: 5 sub-blocks, one per
+// middle code 000 001 010 100 101 in this order, of F(L+2) rows each (F(L+1)
+// where middle bit 0 is set, because low bit L-1 is then clear); a tile whose
+// high bit L + 3 is set has the first three only.  A CTA takes one tile at a
+// time and a thread one low code i and one 16-byte chunk of the row (all
+// vectors of a row are adjacent), for all sub-blocks at once:
 //   - which low bits of i flip, and where to, is the same for every
 //     sub-block and every tile: each thread works it out once per launch,
-//     and per flip one address serves up to 8 shared-memory gathers;
-//   - flips of middle bits are the thread's own registers;
+//     and per flip one address serves up to 5 shared-memory gathers;
+//   - flips of middle bits are the thread's own rows;
 //   - a flip of a high bit moves the whole tile by +- F(k+2) rows: coalesced
-//     reads of x, up to 8 in flight, with one amplitude and one decision for
-//     the tile (the flip of bit L + 4 reaches the first five sub-blocks).
+//     reads of x, up to 10 in flight, with one amplitude and one decision for
+//     the tile (the flip of bit L + 3 reaches the first three sub-blocks).
+// With 4 middle bits (8 sub-blocks) the same code spilled 200 to 800 bytes.
 // One warp decodes the next tile's prefix and its flip list while the CTA
 // works on the current tile.
 //

@@ -17,8 +17,8 @@
 // observables.py:162-205 spin_observables_basis (restricted basis: targets
 // outside the basis drop out), the <n_i n_j> of observables.py:40-47
 // corr_matrix and PauliPlan.expect (observables.py:486-622) for the Pauli
-// strings.  Items come in groups of eight, one group per blockIdx.y; a
-// thread keeps the 24 sums of its group in registers over a grid-stride
+// strings.  Items come in groups of six, one group per blockIdx.y; a
+// thread keeps the 18 sums of its group in registers over a grid-stride
 // loop of rows, so v is read once per group and every flip target once per
 // item.  Block sums go to per-block partials and a second kernel adds them
 // in a fixed order (deterministic results).
