@@ -16,7 +16,8 @@
 // from the step's checkpoint, another 1827 of 7186 phases), a step's last
 // reverse phase also writes lambda and the next step's u_M, and each thread
 // adds up its gradient dots over a step, one block sum per step.  20-site
-// ring, 200 steps, complex64: 22.8 -> 11.0 ms (14.9 with the row values read from memory in each phase).  Four lanes share a row (its
+// ring, 200 steps, complex64: 22.8 -> 10.5 ms (14.9 with the row values read
+// from memory in each phase).  Four lanes share a row (its
 // flips split between them) as in k_adjoint_step, and keep its flip targets
 // in registers across all sweeps; every step's Chebyshev plan (a, b, M, c_m)
 // is computed on the host first and read from device arrays.  Gradient dots
@@ -44,7 +45,6 @@ struct CoopAdj {
   const double *pc;        // [K][Mmax + 1][2] coefficients c_m
   const double *om, *dl;   // [K] Omega_k and -Delta_k
   const S *diagV;          // the V part of the diagonal
-  const double *diag64;
   S ahalf[EL_MAX_SITES];   // a_i / 2 per bit position
   S bsh[EL_MAX_SITES];     // b_i per bit position
   S *ckp;                  // [K + 1][dim] complex checkpoints
@@ -84,6 +84,23 @@ __device__ __forceinline__ void row_flips(const CoopAdj<S> &P, uint64_t code, in
     sim += __shfl_xor_sync(0xffffffffu, sim, off);
     nb += __shfl_xor_sync(0xffffffffu, nb, off);
   }
+}
+
+// The arithmetic of a row.  A complex64 gradient is the result of some
+// thousand FP32 steps, and how each of them rounds shows in its digits (2e-6
+// to 2e-5 between two ways of rounding 200 steps on the 20-site ring), so the
+// order of the roundings is written out here, once for all forms of the
+// gradient (terms stored or formed again, a row in registers or in memory).
+template <typename S>
+__device__ __forceinline__ S mul_re(S ar, S ai, S br, S bi) { return fma(ar, br, -(ai * bi)); }    // Re a b
+template <typename S>
+__device__ __forceinline__ S mul_im(S ar, S ai, S br, S bi) { return fma(ar, bi, ai * br); }       // Im a b
+template <typename S>
+__device__ __forceinline__ S mul_im2(S ar, S ai, S br, S bi) { return fma(ai, br, ar * bi); }      // the same, other product first
+// (alpha H_k + beta) x of one component: h = d x + om s
+template <typename S>
+__device__ __forceinline__ S apply_row(S alpha, S beta, S d, S om, S x, S s) {
+  return fma(beta, x, alpha * fma(om, s, d * x));
 }
 
 // Block sum of two doubles into slot[0..1] (thread 0 writes).
@@ -190,30 +207,29 @@ __device__ __forceinline__ void sweep(const CoopAdj<S> &P, S om, S dl, const Swe
     }
     if (lane != 0 || !active) continue;
     const S xr = W.x[2 * r], xi = W.x[2 * r + 1];
-    const S dsum = P.diagV[r] + dl * nb;
-    const S hre = dsum * xr + om * sre, him = dsum * xi + om * sim;
-    S yre = W.alpha * hre + W.beta * xr, yim = W.alpha * him + W.beta * xi;
+    const S dsum = fma(dl, nb, P.diagV[r]);
+    S yre = apply_row(W.alpha, W.beta, dsum, om, xr, sre), yim = apply_row(W.alpha, W.beta, dsum, om, xi, sim);
     if (W.z) { yre -= W.z[2 * r]; yim -= W.z[2 * r + 1]; }
     if (W.lam) {
       const S lr = W.lam[2 * r], li = W.lam[2 * r + 1];
-      yre += W.clr * lr - W.cli * li;
-      yim += W.clr * li + W.cli * lr;
+      yre += mul_re(W.clr, W.cli, lr, li);
+      yim += mul_im(W.clr, W.cli, lr, li);
     }
     if (W.acc_mode == 3) {
       W.acc[2 * r] = yre;
       W.acc[2 * r + 1] = yim;
-      W.y[2 * r] = W.wr * yre - W.wi * yim;
-      W.y[2 * r + 1] = W.wr * yim + W.wi * yre;
+      W.y[2 * r] = mul_re(W.wr, W.wi, yre, yim);
+      W.y[2 * r + 1] = mul_im(W.wr, W.wi, yre, yim);
     } else {
       W.y[2 * r] = yre;
       W.y[2 * r + 1] = yim;
     }
     if (W.acc_mode == 1) {
-      W.acc[2 * r] = W.w0r * xr - W.w0i * xi + W.wr * yre - W.wi * yim;
-      W.acc[2 * r + 1] = W.w0r * xi + W.w0i * xr + W.wr * yim + W.wi * yre;
+      W.acc[2 * r] = fma(-W.wi, yim, fma(W.wr, yre, mul_re(W.w0r, W.w0i, xr, xi)));
+      W.acc[2 * r + 1] = fma(W.wi, yre, fma(W.wr, yim, mul_im2(W.w0r, W.w0i, xr, xi)));
     } else if (W.acc_mode == 2) {
-      W.acc[2 * r] += W.wr * yre - W.wi * yim;
-      W.acc[2 * r + 1] += W.wr * yim + W.wi * yre;
+      W.acc[2 * r] += mul_re(W.wr, W.wi, yre, yim);
+      W.acc[2 * r + 1] += mul_im2(W.wr, W.wi, yre, yim);
     }
     if (W.t) {
       const double tr = W.t[2 * r], ti = W.t[2 * r + 1];
@@ -228,8 +244,7 @@ __device__ __forceinline__ void sweep(const CoopAdj<S> &P, S om, S dl, const Swe
 // u_{m+1}, u_{m+2}, lambda, its diagonal) stay in registers of the row's first
 // lane, a step's coefficients come through shared memory, and the stored
 // term of the next phase is read before the barrier.  What a phase waits for
-// after its barrier is one round of flip partners.  The row's own values are
-// FP64 also for FP32 vectors: only what is published is rounded.
+// after its barrier is one round of flip partners.
 constexpr int MAXC = 256;   // terms of a step held in shared memory
 
 template <typename S>
@@ -257,43 +272,49 @@ __device__ __forceinline__ void gather_flips(const RowCache<S> &rc, const S *x, 
 template <typename S>
 __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, double *red, unsigned &gen) {
   typedef typename VecT<S, true>::type V2;
-  __shared__ double cbuf[2][2 * MAXC];
+  __shared__ S cbuf[2][2 * MAXC];
   __shared__ double s_ov[2];
   const size_t vs = (size_t)P.B.dim * 2;
   const bool mine = rc.active && (threadIdx.x & (CL - 1)) == 0;   // this thread finishes the row
   const int64_t r = rc.r;
   auto sync = [&]() { coop_sync(P.bar, P.err, P.nctas, P.poll_limit, gen); };
   auto at = [&](const S *p) { return reinterpret_cast<const V2 *>(p)[r]; };
-  auto put = [&](S *p, double re, double im) { V2 v; v.x = (S)re; v.y = (S)im; reinterpret_cast<V2 *>(p)[r] = v; };
+  auto put = [&](S *p, S re, S im) { V2 v; v.x = re; v.y = im; reinterpret_cast<V2 *>(p)[r] = v; };
   // coefficients of step k into buffer k & 1 (read after the next barrier)
   auto fetch = [&](int k) {
     if (k < 0 || k >= P.K) return;
     const double *c = P.pc + (size_t)k * (P.Mmax + 1) * 2;
-    for (int q = threadIdx.x; q < 2 * (P.pm[k] + 1); q += CNT) cbuf[k & 1][q] = c[q];
+    for (int q = threadIdx.x; q < 2 * (P.pm[k] + 1); q += CNT) cbuf[k & 1][q] = (S)c[q];
   };
-  const double diag = P.diag64[r];
+  const S diag = P.diagV[r];
   V2 x0 = at(P.ckp);
-  double xr = x0.x, xi = x0.y;       // own value of the vector the next sweep gathers
+  S xr = x0.x, xi = x0.y;       // own value of the vector the next sweep gathers
   fetch(0);
   __syncthreads();
   // ---- forward
   for (int k = 0; k < P.K; ++k) {
-    const double a = P.pa[k], b = P.pb[k], om = P.om[k];
-    const double d = diag + P.dl[k] * (double)rc.nb;
+    const S a = (S)P.pa[k], b = (S)P.pb[k], om = (S)P.om[k], dl = (S)P.dl[k];
+    const S al1 = S(1) / a, be1 = -b / a, al2 = S(2) / a, be2 = S(-2) * b / a;
+    const S d = fma(dl, rc.nb, diag);
     const int M = P.pm[k];
-    const double *c = cbuf[k & 1];
+    const S *c = cbuf[k & 1];
     S *term = P.term + (size_t)k * (P.Mmax + 1) * vs;
     S *out = P.ckp + (size_t)(k + 1) * vs;
     const S *x = P.ckp + (size_t)k * vs;
-    double zr = 0.0, zi = 0.0;
-    double accr = c[0] * xr - c[1] * xi, acci = c[0] * xi + c[1] * xr;
+    S zr = S(0), zi = S(0), accr = S(0), acci = S(0);
     for (int m = 1; m <= M; ++m) {
       S re, im;
       gather_flips<S>(rc, x, re, im);
-      const double al = (m == 1 ? 1.0 : 2.0) / a, be = (m == 1 ? -b : -2.0 * b) / a;
-      const double yr = al * (d * xr + om * re) + be * xr - zr, yi = al * (d * xi + om * im) + be * xi - zi;
-      accr += c[2 * m] * yr - c[2 * m + 1] * yi;
-      acci += c[2 * m] * yi + c[2 * m + 1] * yr;
+      const S al = m == 1 ? al1 : al2, be = m == 1 ? be1 : be2;
+      const S wr = c[2 * m], wi = c[2 * m + 1];
+      const S yr = apply_row(al, be, d, om, xr, re) - zr, yi = apply_row(al, be, d, om, xi, im) - zi;
+      if (m == 1) {
+        accr = fma(-wi, yi, fma(wr, yr, mul_re(c[0], c[1], xr, xi)));
+        acci = fma(wi, yr, fma(wr, yi, mul_im2(c[0], c[1], xr, xi)));
+      } else {
+        accr += mul_re(wr, wi, yr, yi);
+        acci += mul_im2(wr, wi, yr, yi);
+      }
       zr = xr; zi = xi;
       xr = yr; xi = yi;
       x = term + (size_t)m * vs;
@@ -309,7 +330,7 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
     }
   }
   // ---- objective, lambda_K and u_M of the last step
-  double lr = 0.0, li = 0.0;
+  S lr = S(0), li = S(0);
   {
     double fa = 0.0, fb = 0.0;
     if (mine) {
@@ -329,16 +350,17 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
     if (blockIdx.x == 0 && threadIdx.x == 0) { P.fout[0] = s_ov[0]; P.fout[1] = s_ov[1]; }
     if (P.target) {   // lambda = <target, psi> target
       const V2 t = at(P.target);
-      lr = s_ov[0] * t.x - s_ov[1] * t.y;
-      li = s_ov[0] * t.y + s_ov[1] * t.x;
+      lr = mul_re((S)s_ov[0], (S)s_ov[1], t.x, t.y);
+      li = mul_im2((S)s_ov[0], (S)s_ov[1], t.x, t.y);
     } else {          // lambda = O psi
-      lr = P.obs[r] * xr;
-      li = P.obs[r] * xi;
+      const S o = (S)P.obs[r];
+      lr = o * xr;
+      li = o * xi;
     }
-    const double *c = cbuf[(P.K - 1) & 1];
+    const S *c = cbuf[(P.K - 1) & 1];
     const int M = P.pm[P.K - 1];
-    xr = c[2 * M] * lr + c[2 * M + 1] * li;       // conj(c_M) lambda
-    xi = c[2 * M] * li - c[2 * M + 1] * lr;
+    xr = mul_re(c[2 * M], -c[2 * M + 1], lr, li);     // conj(c_M) lambda
+    xi = mul_im(c[2 * M], -c[2 * M + 1], lr, li);
     if (mine) put(P.U, xr, xi);
     fetch(P.K - 2);
     sync();
@@ -346,12 +368,13 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
   // ---- backward
   int us = 0;
   for (int k = P.K - 1; k >= 0; --k) {
-    const double a = P.pa[k], b = P.pb[k], om = P.om[k];
-    const double d = diag + P.dl[k] * (double)rc.nb;
+    const S a = (S)P.pa[k], b = (S)P.pb[k], om = (S)P.om[k], dl = (S)P.dl[k];
+    const S al1 = S(1) / a, be1 = -b / a, al2 = S(2) / a, be2 = S(-2) * b / a;
+    const S d = fma(dl, rc.nb, diag);
     const int M = P.pm[k], Mn = k > 0 ? P.pm[k - 1] : 0;
-    const double *c = cbuf[k & 1], *cn = cbuf[(k & 1) ^ 1];
+    const S *c = cbuf[k & 1], *cn = cbuf[(k & 1) ^ 1];
     const S *term = P.term + (size_t)k * (P.Mmax + 1) * vs;
-    double zr = 0.0, zi = 0.0;
+    S zr = S(0), zi = S(0);
     double gO = 0.0, gD = 0.0;
     if (M == 1 && k + 1 < P.K) {   // one phase: the next step's coefficients are needed in it
       fetch(k - 1);
@@ -361,14 +384,15 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
     for (int m = M - 1; m >= 0; --m) {
       S re, im;
       gather_flips<S>(rc, P.U + (size_t)us * vs, re, im);
-      const double al = (m == 0 ? 1.0 : 2.0) / a, be = (m == 0 ? -b : -2.0 * b) / a;
+      const S al = m == 0 ? al1 : al2, be = m == 0 ? be1 : be2;
+      const S clr = c[2 * m], cli = -c[2 * m + 1];
       // conj(c_m) lambda + (s/a)(H - b) u_{m+1} - u_{m+2}
-      const double yr = al * (d * xr + om * re) + be * xr - zr + (c[2 * m] * lr + c[2 * m + 1] * li);
-      const double yi = al * (d * xi + om * im) + be * xi - zi + (c[2 * m] * li - c[2 * m + 1] * lr);
+      const S yr = apply_row(al, be, d, om, xr, re) - zr + mul_re(clr, cli, lr, li);
+      const S yi = apply_row(al, be, d, om, xi, im) - zi + mul_im(clr, cli, lr, li);
       if (mine) {
         const double w = (m == 0) ? 1.0 : 2.0, tr = t.x, ti = t.y;
-        gO += w * ((double)re * tr + (double)im * ti);                       // Re(conj(G_O u) t)
-        gD -= w * (double)rc.nb * ((double)xr * tr + (double)xi * ti);       // Re(conj(G_D u) t)
+        gO += w * ((double)re * tr + (double)im * ti);                                  // Re(conj(G_O u) t)
+        gD -= w * (double)rc.nb * ((double)xr * tr + (double)xi * ti);                  // Re(conj(G_D u) t)
       }
       us = us == 2 ? 0 : us + 1;
       zr = xr; zi = xi;
@@ -379,8 +403,8 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
       } else {   // lambda_{k-1} = u_0, published as u_M of step k - 1
         lr = yr;
         li = yi;
-        xr = cn[2 * Mn] * lr + cn[2 * Mn + 1] * li;
-        xi = cn[2 * Mn] * li - cn[2 * Mn + 1] * lr;
+        xr = mul_re(cn[2 * Mn], -cn[2 * Mn + 1], lr, li);
+        xi = mul_im(cn[2 * Mn], -cn[2 * Mn + 1], lr, li);
         block_sum2(gO, gD, red, P.part + ((size_t)k * P.nctas + blockIdx.x) * 2);
       }
       if (mine) put(P.U + (size_t)us * vs, xr, xi);
@@ -390,9 +414,9 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
   }
 }
 
-template <typename S>
 // At most 128 registers: the pulse problems' bases then fit one pass of the
 // grid, which the register cache of the rows needs.
+template <typename S>
 __global__ void __launch_bounds__(CNT, 1) k_adjoint_coop(const CoopAdj<S> P) {
   __shared__ double red[2 * (CNT / 32)];
   __shared__ double s_ov[2];
@@ -468,8 +492,8 @@ __global__ void __launch_bounds__(CNT, 1) k_adjoint_coop(const CoopAdj<S> P) {
       S lr, li;
       if (P.target) {   // lambda = <target, psi> target
         const S tr = P.target[2 * r], ti = P.target[2 * r + 1];
-        lr = ovr * tr - ovi * ti;
-        li = ovr * ti + ovi * tr;
+        lr = mul_re(ovr, ovi, tr, ti);
+        li = mul_im2(ovr, ovi, tr, ti);
       } else {          // lambda = O psi
         const S o = (S)P.obs[r];
         lr = o * psi[2 * r];
@@ -477,8 +501,8 @@ __global__ void __launch_bounds__(CNT, 1) k_adjoint_coop(const CoopAdj<S> P) {
       }
       P.lam[2 * r] = lr;
       P.lam[2 * r + 1] = li;
-      P.U[2 * r] = cr * lr - ci * li;       // u_M = conj(c_M) lambda of the last step
-      P.U[2 * r + 1] = cr * li + ci * lr;
+      P.U[2 * r] = mul_re(cr, ci, lr, li);       // u_M = conj(c_M) lambda of the last step
+      P.U[2 * r + 1] = mul_im(cr, ci, lr, li);
     }
     sync();
   }
@@ -594,7 +618,6 @@ int adjoint_coop(el_ctx *ctx, el_ham *h, int K, const std::vector<ChebPlan> &pla
   P.pa = d_pa; P.pb = d_pb; P.pm = d_pm; P.pc = d_pc; P.om = d_om; P.dl = d_dl;
   if (std::is_same<S, float>::value) { int rc = el::ham_diag32(ctx, h); if (rc) return rc; }
   P.diagV = std::is_same<S, float>::value ? (const S *)(void *)h->d_diagV32 : (const S *)(void *)h->d_diagV64;
-  P.diag64 = h->d_diagV64;
   for (int q = 0; q < n; ++q) {
     P.ahalf[q] = (S)(0.5 * ash[n - 1 - q]);
     P.bsh[q] = (S)bsh[n - 1 - q];
