@@ -1,22 +1,14 @@
 """complex64 pulse gradient against the same recurrence restated in FP32 on the
 CPU, rounding by rounding: forward terms t_m, accumulated states, lambda and
 the reverse terms u_m, so that a change in how a row is rounded shows at once
-and not only as digits lost over some hundred steps.  Fused multiply-adds are
-formed in extended precision and rounded once."""
+and not only as digits lost over some hundred steps."""
 import numpy as np
 import pytest
 
 from energy_level_b200 import configs
+from fp32_restated import chebyshev_plan, f4, fma
 
 pytestmark = pytest.mark.gpu
-
-CONV = 2.0 * np.pi * 1e-3
-f4 = np.float32
-
-
-def fma(a, b, c):
-    return (np.asarray(a, np.longdouble) * np.asarray(b, np.longdouble) + np.asarray(c, np.longdouble)).astype(f4)
-
 
 def _cmul(a, z, first=True):
     """a z with the roundings of a row: first picks which product of the
@@ -26,19 +18,10 @@ def _cmul(a, z, first=True):
     return re, im
 
 
-def _plan(V, flips, occ, tau, om, de, tol=1e-7):
-    from scipy.special import jv
+def _plan(V, flips, occ, tau, om, de):
     R = 0.5 * abs(om) * flips
     d = V - de * occ
-    lo, hi = (d - R).min(), (d + R).max()
-    a, b = max(0.5 * (hi - lo) * (1.0 + 1e-6), 1e-12), 0.5 * (hi + lo)
-    x, phi = a * CONV * tau, b * CONV * tau
-    mmax = int(x + 30.0 + 6.0 * np.cbrt(x + 1.0))
-    J = jv(np.arange(mmax + 1), x)
-    over = [m for m in range(1, mmax + 1) if 2.0 * abs(J[m]) > 0.25 * tol]
-    M = min(over[-1] + 1, mmax) if over else 1
-    m = np.arange(M + 1)
-    c = np.where(m == 0, 1.0, 2.0) * J[:M + 1] * np.array([1, -1j, -1, 1j])[m & 3] * np.exp(-1j * phi)
+    a, b, M, c = chebyshev_plan((d - R).min(), (d + R).max(), tau)
     return a, b, M, c.real.astype(f4), c.imag.astype(f4)
 
 
