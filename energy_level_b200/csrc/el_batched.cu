@@ -1166,6 +1166,21 @@ __global__ void k_batch_diag(int count, const Inst *inst, const double *Vmats, c
   }
 }
 
+// Lets fn use all dynamic shared memory that a block can have beside its
+// static part.  The limit belongs to the function on the device, not to a
+// context, and contexts are one per thread, so it is the same for every batch:
+// a limit of this batch's size could be lowered by another thread's batch
+// before this one's launch.
+int dynamic_smem_limit(el_ctx *ctx, const void *fn, int64_t *most) {
+  int block = 0;
+  EL_CUDA_TRY(ctx, cudaDeviceGetAttribute(&block, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  cudaFuncAttributes fa;
+  EL_CUDA_TRY(ctx, cudaFuncGetAttributes(&fa, fn));
+  *most = block - (int64_t)fa.sharedSizeBytes;
+  EL_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*most));
+  return EL_OK;
+}
+
 uint64_t fibh(int i) { uint64_t a = 0, b = 1; for (int k = 0; k < i; ++k) { uint64_t t = a + b; a = b; b = t; } return a; }
 
 struct el_batch_impl {
@@ -1439,18 +1454,19 @@ int el_batch_run(el_ctx *ctx, el_batch *b, int threads, int ctas_per_sm, uint64_
   A.iters = b->d_iout; A.conv = b->d_iout + b->count;
   A.nat = b->want_nat ? b->d_nat : nullptr;
   // shared memory for the largest vector, or what the CTAs of an SM leave
-  int smem_sm = 0, smem_block = 0;
+  int smem_sm = 0;
   EL_CUDA_TRY(ctx, cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
-  EL_CUDA_TRY(ctx, cudaDeviceGetAttribute(&smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
   auto launch = [&](const void *fn) -> int {
+    int64_t most = 0;
+    const int rc = dynamic_smem_limit(ctx, fn, &most);
+    if (rc) return rc;
     cudaFuncAttributes fa;
     EL_CUDA_TRY(ctx, cudaFuncGetAttributes(&fa, fn));
     // 1 KB per CTA is the system's
-    const int64_t room = std::min<int64_t>(smem_sm / ctas_per_sm - 1024, smem_block) - (int64_t)fa.sharedSizeBytes;
+    const int64_t room = std::min<int64_t>(smem_sm / ctas_per_sm - 1024 - (int64_t)fa.sharedSizeBytes, most);
     const int64_t rows = std::max<int64_t>(0, std::min<int64_t>(room / (int64_t)es, b->dim_max));
     A.smem_rows = rows;
     const size_t smem = (size_t)rows * es;
-    EL_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void *kargs[] = {(void *)&A};
     EL_CUDA_TRY(ctx, cudaLaunchKernel(fn, dim3(grid), dim3(threads), kargs, smem, ctx->stream));
     return EL_OK;
@@ -1541,7 +1557,10 @@ int el_batch_run_coop(el_ctx *ctx, el_batch *b, int reorth_passes, int check_eve
     }
     if (b->dtype == EL_F32) { EL_CPICK(float) } else { EL_CPICK(double) }
 #undef EL_CPICK
-    EL_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
+    int64_t most = 0;
+    const int rc = dynamic_smem_limit(ctx, fn, &most);
+    if (rc) return rc;
+    if ((int64_t)P.smem > most) return fail(ctx, EL_EINVAL, "cooperative solver needs %zu bytes of shared memory", P.smem);
     int per_sm = 0;
     const int threads = P.nt * coop_tp(P.nt);
     EL_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, P.smem));
