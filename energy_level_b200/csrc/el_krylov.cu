@@ -96,9 +96,11 @@ extern "C" int el_bounds(el_ctx *ctx, el_ham *h, int max_iter, double tol,
   // few at a time and the host reads their scalars together: on 121,393 rows
   // (57 steps) the two waits per step cost more than the step's kernels.
   const int maxit = (int)std::min<int64_t>(max_iter, dim);
-  double *rec = (double *)el::workspace(ctx, 16, (size_t)(maxit + 1) * 4 * sizeof(double));
-  if (!rec) return EL_ENOMEM;
   const int ahead = plan ? 1 : steps_ahead(vb);
+  // a step reads the one before it: two rounds of queued steps, in turn
+  double *const recs = (double *)el::workspace(ctx, 16, 2 * (size_t)ahead * 4 * sizeof(double));
+  if (!recs) return EL_ENOMEM;
+  auto rec = [&](int q) { return recs + 4 * (q % (2 * ahead)); };
   double kappa = 1.0, kappa_prev = 1.0;
   int stable = 0;
   bool done = false;
@@ -114,11 +116,11 @@ extern "C" int el_bounds(el_ctx *ctx, el_ham *h, int max_iter, double tol,
         ApplyArgs A;
         memset(&A, 0, sizeof A);
         A.dtype = dtype; A.nvec = 1; A.x = v; A.z = vp; A.y = w;
-        A.a = 1.0; A.b = 0.0; A.c_dev = q ? rec + 4 * (q - 1) + 2 : nullptr; A.dots = d_sc; A.want_dots = 7;
+        A.a = 1.0; A.b = 0.0; A.c_dev = q ? rec(q - 1) + 2 : nullptr; A.dots = d_sc; A.want_dots = 7;
         rc = el::launch_apply(ctx, h, A);
       }
       if (rc) return rc;
-      rc = el::launch_lanczos_update(ctx, dtype, dim, v, w, d_sc, q ? rec + 4 * (q - 1) + 1 : d_one, rec + 4 * q);
+      rc = el::launch_lanczos_update(ctx, dtype, dim, v, w, d_sc, q ? rec(q - 1) + 1 : d_one, rec(q));
       if (rc) return rc;
       // s_{j-1} <- s_j ; s_j <- s_{j+1}
       std::swap(vp, v);
@@ -127,7 +129,7 @@ extern "C" int el_bounds(el_ctx *ctx, el_ham *h, int max_iter, double tol,
       std::swap(iv, iw);
     }
     hr.resize(4 * nb);
-    rc = sync_read(ctx, rec + 4 * j, 4 * nb, hr.data());
+    rc = sync_read(ctx, rec(j), 4 * nb, hr.data());   // j is a multiple of ahead: one piece
     if (rc) return rc;
     for (int q = 0; q < nb && !done; ++q, ++j) {
       const double alpha = hr[4 * q], n2 = hr[4 * q + 1], bpred = hr[4 * q + 3];
