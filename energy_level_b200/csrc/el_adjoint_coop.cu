@@ -279,6 +279,8 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
   const int64_t r = rc.r;
   auto sync = [&]() { coop_sync(P.bar, P.err, P.nctas, P.poll_limit, gen); };
   auto at = [&](const S *p) { return reinterpret_cast<const V2 *>(p)[r]; };
+  // of the caller's target, which need only be aligned to one value
+  auto at_any = [&](const S *p) { V2 v; v.x = p[2 * r]; v.y = p[2 * r + 1]; return v; };
   auto put = [&](S *p, S re, S im) { V2 v; v.x = re; v.y = im; reinterpret_cast<V2 *>(p)[r] = v; };
   // coefficients of step k into buffer k & 1 (read after the next barrier)
   auto fetch = [&](int k) {
@@ -335,7 +337,7 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
     double fa = 0.0, fb = 0.0;
     if (mine) {
       if (P.target) {
-        const V2 t = at(P.target);
+        const V2 t = at_any(P.target);
         fa = (double)t.x * xr + (double)t.y * xi;   // conj(target) psi
         fb = (double)t.x * xi - (double)t.y * xr;
       } else {
@@ -349,7 +351,7 @@ __device__ void gradient_one_pass(const CoopAdj<S> &P, const RowCache<S> &rc, do
     block_sum2(sa, sb, red, s_ov);
     if (blockIdx.x == 0 && threadIdx.x == 0) { P.fout[0] = s_ov[0]; P.fout[1] = s_ov[1]; }
     if (P.target) {   // lambda = <target, psi> target
-      const V2 t = at(P.target);
+      const V2 t = at_any(P.target);
       lr = mul_re((S)s_ov[0], (S)s_ov[1], t.x, t.y);
       li = mul_im2((S)s_ov[0], (S)s_ov[1], t.x, t.y);
     } else {          // lambda = O psi
