@@ -367,44 +367,21 @@ __global__ void __launch_bounds__(256) k_apply_hop(BasisDev B, HamArgs<S> H, KAr
 // the block so that every lane reaches the shuffles; lanes past the last row
 // work on row 0 and store nothing.
 
+// A row's value in one access: W = 2 for a complex one (aligned to both parts).
+template <typename S, int W>
+struct alignas(W * sizeof(S)) RowValue { S s[W]; };
 template <typename S, int W>
 __device__ __forceinline__ void ld_row(const S *p, S (&v)[W]) {
-  constexpr int BYTES = W * (int)sizeof(S);
-  if constexpr (BYTES % 16 == 0) {
-    union { uint4 u[BYTES / 16]; S s[W]; } t;
+  const RowValue<S, W> t = *reinterpret_cast<const RowValue<S, W> *>(p);
 #pragma unroll
-    for (int i = 0; i < BYTES / 16; ++i) t.u[i] = reinterpret_cast<const uint4 *>(p)[i];
-#pragma unroll
-    for (int i = 0; i < W; ++i) v[i] = t.s[i];
-  } else if constexpr (BYTES == 8) {
-    union { uint2 u; S s[W]; } t;
-    t.u = *reinterpret_cast<const uint2 *>(p);
-#pragma unroll
-    for (int i = 0; i < W; ++i) v[i] = t.s[i];
-  } else {
-#pragma unroll
-    for (int i = 0; i < W; ++i) v[i] = p[i];
-  }
+  for (int i = 0; i < W; ++i) v[i] = t.s[i];
 }
-
 template <typename S, int W>
 __device__ __forceinline__ void st_row(S *p, const S (&v)[W]) {
-  constexpr int BYTES = W * (int)sizeof(S);
-  if constexpr (BYTES % 16 == 0) {
-    union { uint4 u[BYTES / 16]; S s[W]; } t;
+  RowValue<S, W> t;
 #pragma unroll
-    for (int i = 0; i < W; ++i) t.s[i] = v[i];
-#pragma unroll
-    for (int i = 0; i < BYTES / 16; ++i) reinterpret_cast<uint4 *>(p)[i] = t.u[i];
-  } else if constexpr (BYTES == 8) {
-    union { uint2 u; S s[W]; } t;
-#pragma unroll
-    for (int i = 0; i < W; ++i) t.s[i] = v[i];
-    *reinterpret_cast<uint2 *>(p) = t.u;
-  } else {
-#pragma unroll
-    for (int i = 0; i < W; ++i) p[i] = v[i];
-  }
+  for (int i = 0; i < W; ++i) t.s[i] = v[i];
+  *reinterpret_cast<RowValue<S, W> *>(p) = t;
 }
 
 // Code of `row` (FULL / CHAIN / RING) in CT arithmetic.
@@ -462,7 +439,6 @@ __global__ void __launch_bounds__(256) k_apply_row(BasisDev B, HamArgs<S> H, KAr
   static_assert(32 % G == 0, "lanes per row: G divides 32");
   typedef uint32_t CT;
   typedef int32_t RT;
-  constexpr int NV = 1;
   constexpr int W = C ? 2 : 1;
   constexpr int U = 8;   // one round covers 8 G sites
   const int n = B.n;
@@ -529,18 +505,14 @@ __global__ void __launch_bounds__(256) k_apply_row(BasisDev B, HamArgs<S> H, KAr
         if (!ok[u]) continue;
         if constexpr (C) {
           if (H.real_amp) {   // uniform: a real drive needs two FMAs per complex entry
-#pragma unroll
-            for (int v = 0; v < 2 * NV; ++v) h[v] += ar[u] * xv[u][v];
+            h[0] += ar[u] * xv[u][0];
+            h[1] += ar[u] * xv[u][1];
           } else {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-              h[2 * v] += ar[u] * xv[u][2 * v] - ai[u] * xv[u][2 * v + 1];
-              h[2 * v + 1] += ar[u] * xv[u][2 * v + 1] + ai[u] * xv[u][2 * v];
-            }
+            h[0] += ar[u] * xv[u][0] - ai[u] * xv[u][1];
+            h[1] += ar[u] * xv[u][1] + ai[u] * xv[u][0];
           }
         } else {
-#pragma unroll
-          for (int v = 0; v < NV; ++v) h[v] += ar[u] * xv[u][v];
+          h[0] += ar[u] * xv[u][0];
         }
       }
     }
@@ -575,14 +547,10 @@ __global__ void __launch_bounds__(256) k_apply_row(BasisDev B, HamArgs<S> H, KAr
       ld_row<S, W>(ap, av);
       const S wr = (S)K.w_re, wi = (S)K.w_im;
       if constexpr (C) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          av[2 * v] += wr * yv[2 * v] - wi * yv[2 * v + 1];
-          av[2 * v + 1] += wr * yv[2 * v + 1] + wi * yv[2 * v];
-        }
+        av[0] += wr * yv[0] - wi * yv[1];
+        av[1] += wr * yv[1] + wi * yv[0];
       } else {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) av[v] += wr * yv[v];
+        av[0] += wr * yv[0];
       }
       st_row<S, W>(ap, av);
     }
@@ -1160,7 +1128,7 @@ namespace {
 // kernels' (tile, barrier, gathers).  Full basis, complex128: n = 14 4.5
 // against 6.3 us, 15 6.2 against 6.5, 16 10.3 against 7.2.  Chains, float64:
 // n = 18 4.7 against 8.3, 22 8.3 against 10.3, 23 (75,025 rows) 10.3 both.
-constexpr int64_t ROW_FULL = 1 << 16, ROW_SECTOR = 148 * 512;
+constexpr int64_t ROW_FULL = 1 << 16, ROW_SECTOR = 75776;
 constexpr int ROW_LANES = 4;
 
 bool row_kernel_ok(const el_ham *h, const ApplyArgs &A) {
@@ -1247,7 +1215,7 @@ int launch_apply(el_ctx *ctx, el_ham *h, const ApplyArgs &A) {
     if (rc) return rc;
   }
   if (row_kernel_ok(h, A)) return launch_apply_row(ctx, h, A, B, K);
-  if (chain_block_ok(h, A)) return launch_chain_block(ctx, h, A, B, K);
+  if (chain_block_ok(ctx, h, A)) return launch_chain_block(ctx, h, A, B, K);
   if (full_block_ok(h, A)) return launch_full_block(ctx, h, A, K);
   if (table_block_ok(h, A)) return launch_table_block(ctx, h, A, B, K);
   if (!h->px.empty() && (B.layout == EL_LAYOUT_FULL || B.layout == EL_LAYOUT_TABLE) && B.n <= 32 &&

@@ -11,10 +11,10 @@ struct HamArgs {
   S delta[EL_MAX_SITES];
   S up_re[EL_MAX_SITES];  // amplitude into a row whose bit k is 1: Omega/2
   S up_im[EL_MAX_SITES];  // (into a row whose bit k is 0: conj(Omega)/2)
-  const ExPair *px;       // exchange channels (generic kernel only)
+  const ExPair *px;       // exchange channels (generic and hop kernels)
   int npx;
-  int lossy;              // loss diagonal present (generic kernel only)
-  int real_amp;           // every sigma^x amplitude is real (row kernel: cheaper complex FMAs)
+  int lossy;              // loss diagonal present (generic and hop kernels)
+  int real_amp;           // every sigma^x amplitude is real: cheaper complex multiply-adds
   S loss[EL_MAX_SITES];   // imaginary diagonal per set bit: -gamma/2 (evolution units)
 };
 
@@ -56,7 +56,7 @@ inline HamArgs<S> ham_args(const el_ham *h, const S *diagV) {
 }
 
 // y = a H x + b x + c z (+ acc, dots) on CHAIN and RING sectors (el_chain.cu).
-bool chain_block_ok(const el_ham *h, const ApplyArgs &A);
+bool chain_block_ok(const el_ctx *ctx, const el_ham *h, const ApplyArgs &A);
 int launch_chain_block(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const BasisDev &B, const KArgs &K);
 
 // The same on the full 2^n basis (el_full.cu).

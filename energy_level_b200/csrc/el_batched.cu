@@ -9,8 +9,8 @@
 // Vectors are FP32 (or FP64); alpha/beta, the omega recurrence of partial
 // reorthogonalisation (Simon 1984) and the tridiagonal eigensolve are FP64.
 // The two lowest Ritz values come from a warp-parallel Sturm multisection;
-// the residual estimate beta_{j+1} |s_j| of the lowest pair from inverse
-// iteration on one thread.  Convergence: residual estimate of both pairs
+// the residual estimate beta_{j+1} |s_j| of either pair from inverse
+// iteration by one warp.  Convergence: residual estimate of both pairs
 // <= tol * max(1, |theta|).  H follows channels.py:58-132 (diagonal
 // delta n + V n n, sigma^x with Omega/2) on nearest-neighbour chain / ring
 // blockade sectors (Zeckendorf ranking), full bases, or the blockade sector
@@ -18,7 +18,7 @@
 // list, and a flip table of target rows built once at set-up); this is the batched
 // counterpart of the reference's dense batched_ground_state
 // (equilibrium.py:251-311) and of per-instance eigsh calls (eq_route.py:540).
-#include "el_internal.cuh"
+#include "el_coop.cuh"
 
 #include <algorithm>
 #include <numeric>
@@ -777,27 +777,6 @@ struct CoopArgs {
   double *nat;                  // [count][MAXN] ground-state <n_k>, or null
 };
 
-__device__ __forceinline__ void grid_barrier(const CoopArgs &G, unsigned &gen) {
-  __syncthreads();
-  gen += (unsigned)G.nctas;
-  if (threadIdx.x == 0) {
-    // release this CTA's writes with the arrival, acquire the others' with
-    // the poll that sees the count complete
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(G.bar) : "memory");
-    if (!*(volatile int *)G.err) {
-      int polls = 0;
-      unsigned v;
-      for (;;) {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(G.bar) : "memory");
-        if (v >= gen) break;
-        if (++polls > G.poll_limit) { atomicExch(G.err, 1); break; }
-        if ((polls & 255) == 0 && *(volatile int *)G.err) break;
-      }
-    }
-  }
-  __syncthreads();
-}
-
 // Dynamic shared memory of the cooperative kernel: the Krylov slice
 // [m + 1][NT + 1] then two inverse-iteration buffers.
 __host__ __device__ inline size_t coop_slice_bytes(int m, int nt, int es) {
@@ -882,6 +861,7 @@ __global__ void __launch_bounds__(NT * coop_tp(NT), 1) k_lanczos_coop(const Coop
   // inverse-iteration buffers of the two Ritz pairs follow the slice in dynamic memory
   double *work = reinterpret_cast<double *>(coop_smem + coop_slice_bytes(m, NT, (int)sizeof(T)));
   unsigned gen = 0;
+  auto barrier = [&]() { el::coop_sync(G.bar, G.err, G.nctas, G.poll_limit, gen); };
   int slot = 0;
   auto part = [&](int sl, int c, int k) -> double * {
     return G.part + ((size_t)sl * G.nctas + c) * (MAXIT + 2) + k;
@@ -891,7 +871,7 @@ __global__ void __launch_bounds__(NT * coop_tp(NT), 1) k_lanczos_coop(const Coop
   // lanes over CTAs, fixed tree) into tot, then every CTA reads tot: two
   // barriers, O(nk) loads per CTA instead of O(nk x G)
   auto reduce_all = [&](int nk) {
-    grid_barrier(G, gen);
+    barrier();
     const int lane = tid & 31, warp = tid >> 5;
     double *tt = G.tot + (size_t)slot * (MAXIT + 2);
     for (int k = blockIdx.x + warp * G.nctas; k < nk; k += G.nctas * (NTH / 32)) {
@@ -900,7 +880,7 @@ __global__ void __launch_bounds__(NT * coop_tp(NT), 1) k_lanczos_coop(const Coop
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
       if (lane == 0) tt[k] = v;
     }
-    grid_barrier(G, gen);
+    barrier();
     for (int k = tid; k < nk; k += NTH) cs[k] = __ldcg(&tt[k]);
     slot ^= 1;
     __syncthreads();
@@ -927,7 +907,7 @@ __global__ void __launch_bounds__(NT * coop_tp(NT), 1) k_lanczos_coop(const Coop
     if (lead) Vs[rt] = valid ? v : (T)0;
     if (lead && valid) vpub[row] = v;
   }
-  grid_barrier(G, gen);
+  barrier();
   int steps = 0;
   double bnext = 0.0, anorm = 0.0;
   for (int j = 0; j < m; ++j) {
@@ -1058,7 +1038,7 @@ __global__ void __launch_bounds__(NT * coop_tp(NT), 1) k_lanczos_coop(const Coop
     const T vn = (T)(w / bnext);
     if (lead) Vs[(size_t)(j + 1) * PITCH + rt] = valid ? vn : (T)0;
     if (lead && valid) vpub[row] = vn;
-    grid_barrier(G, gen);
+    barrier();
   }
   if (G.nat) {
     // site occupations of the ground-state Ritz vector (as in the batched

@@ -339,7 +339,7 @@ k_chain_block(const __grid_constant__ ChainGeom G, const __grid_constant__ HamAr
 // complex64 vector, n = 31: 64.7 us at L = 9, 62.2 at 10, 60.6 at 11; 512
 // threads at L = 12 measured 81); smaller ones keep two tiles per SM on
 // short chains.  Returns 0 where no L gives a tile.
-int chain_low_bits(const ChainGeom &g, const BasisDev &B, int nch) {
+int chain_low_bits(const ChainGeom &g, const BasisDev &B, int nch, int sms) {
   const int nmin = g.nseg == 2 ? g.nbits[1] : g.nbits[0];
   int best = 0;
   for (int L = 3; L + MID + 1 <= nmin && L <= 16; ++L) {
@@ -347,13 +347,13 @@ int chain_low_bits(const ChainGeom &g, const BasisDev &B, int nch) {
     int64_t tiles = 0;
     for (int s = 0; s < g.nseg; ++s) tiles += (int64_t)B.fib[g.nbits[s] - L - MID + 2];
     if (threads > SUB) break;
-    if (best && tiles < 2 * 148) break;
+    if (best && tiles < 2 * sms) break;
     best = L;
   }
   return best;
 }
 
-bool chain_geom(const el_ham *h, const ApplyArgs &A, const BasisDev &B, ChainGeom *g) {
+bool chain_geom(const el_ctx *ctx, const el_ham *h, const ApplyArgs &A, const BasisDev &B, ChainGeom *g) {
   memset(g, 0, sizeof *g);
   const int n = h->n;
   memcpy(g->fib, B.fib, sizeof g->fib);
@@ -371,7 +371,7 @@ bool chain_geom(const el_ham *h, const ApplyArgs &A, const BasisDev &B, ChainGeo
   g->nch = chunks_per_row(A);
   if (g->nch > 32) return false;
   while ((1 << g->lognch) < g->nch) ++g->lognch;
-  g->L = chain_low_bits(*g, B, g->nch);
+  g->L = chain_low_bits(*g, B, g->nch, sm_count(ctx));
   if (!g->L) return false;
   for (int k = 0; k < n; ++k)
     if (h->om_re[k] != 0.0 || h->om_im[k] != 0.0) g->amps |= 1ULL << k;
@@ -426,16 +426,16 @@ int launch_block_c(el_ctx *ctx, const ChainGeom &G, const HamArgs<S> &H, const K
 
 namespace el {
 
-bool chain_block_ok(const el_ham *h, const ApplyArgs &A) {
+bool chain_block_ok(const el_ctx *ctx, const el_ham *h, const ApplyArgs &A) {
   if (!h->px.empty() || h->lossy) return false;   // sigma^x channels and a real diagonal only
   if (!chunks_aligned(A)) return false;
   ChainGeom G;
-  return chain_geom(h, A, basis_dev(h->basis), &G);
+  return chain_geom(ctx, h, A, basis_dev(h->basis), &G);
 }
 
 int launch_chain_block(el_ctx *ctx, el_ham *h, const ApplyArgs &A, const BasisDev &B, const KArgs &K) {
   ChainGeom G;
-  if (!chain_geom(h, A, B, &G)) return fail(ctx, EL_EINVAL, "no chain tile for this shape");
+  if (!chain_geom(ctx, h, A, B, &G)) return fail(ctx, EL_EINVAL, "no chain tile for this shape");
   const int n = h->n, nv = A.nvec;
   switch (A.dtype) {
     case EL_F32: {

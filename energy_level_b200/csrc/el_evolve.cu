@@ -9,7 +9,8 @@
 // (the Jacobi-Anger expansion), multiplied by the global phase
 // exp(-i b CONV tau).  Bessel values J_m(x) come from Miller's backward
 // recurrence normalised by J_0 + 2 sum J_2k = 1.  The series is cut when the
-// remaining coefficients fall below `tol`.  Each term is one fused kernel:
+// remaining coefficients fall below `tol`.  Each term is one fused kernel (or,
+// on full bases of 5 to 18 sites, the whole step: el_cheb_coop.cu):
 //     t_{m+1} = (2/a) H t_m - (2b/a) t_m - t_{m-1},  acc += c_{m+1} t_{m+1}.
 #include "el_internal.cuh"
 

@@ -9,7 +9,7 @@
 // class and then the rank.  Four flips are looked up, gathered and added at a
 // time: the look-ups are a chain of two or three reads from L1 or L2, and what
 // bounds the kernel is how many of these chains are in flight.  5 x 6 lattice
-// (470,832 rows), float64: 39 us one flip after the other with 64-bit codes,
+// (454,385 rows), float64: 39 us one flip after the other with 64-bit codes,
 // 28.5 us here; 16 float32 vectors 434 -> 74.
 #include "el_tile.cuh"
 
