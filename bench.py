@@ -1033,17 +1033,18 @@ def native_adjoint20(h, args):
                      {"n_sites": n, "basis": "ring nearest-neighbour blockade sector", "dim": p32.basis.dim,
                       "pulse_steps": len(tau), "T_ns": float(np.sum(tau)), "objective": "|<Z2|psi(T)>|^2",
                       "parameters": 2 * len(tau), "form": "adjoint through the Chebyshev steps, complex64, "
-                      "terms recomputed per step", "l2": "dim 15,127: L2-resident (latency-bound)"})
-    # sweeps of one gradient: the launches of the launch-per-term schedule
-    # (each is one sweep of a Chebyshev or reverse term over the basis:
-    # state, two recurrence vectors, adjoint, accumulator -- 5 complex64
-    # vectors -- and the FP32 diagonal); the chosen schedule runs the same
-    # sweeps as phases of one cooperative launch
+                      "every step's terms stored", "l2": "dim 15,127: L2-resident (latency-bound)"})
+    # sweeps that a gradient cannot do without: every forward and every
+    # reverse term once (each over state, two recurrence vectors, adjoint,
+    # accumulator -- 5 complex64 vectors -- and the FP32 diagonal), as phases
+    # of one cooperative launch.  Counted from the launch-per-term schedule,
+    # which forms the forward terms of a step again in the reverse pass:
+    # 3 M + 1 launches for a step of M terms, and 5 for the whole gradient
     p32.set_schedule("stream")
     l0 = h.ctx.launches
     p32.evaluate(tau, om, Delta)
     torch.cuda.synchronize()
-    sweeps = h.ctx.launches - l0
+    sweeps = 2 * ((h.ctx.launches - l0 - 5 - len(tau)) // 3)
     p32.set_schedule("auto")
     rl = roofline(sweeps * p32.basis.dim * (5 * 8 + 4), el / steps,
                   kernel="k_adjoint_coop (the whole gradient: %d sweeps as phases of one cooperative launch)" % sweeps)

@@ -275,7 +275,7 @@ int step_bounds(el_ctx *ctx, el_ham *h, int K, const double *omega_k, const doub
   memset(&sh, 0, sizeof sh);
   for (int q = 0; q < n; ++q) { sh.a[q] = ash[n - 1 - q]; sh.b[q] = bsh[n - 1 - q]; }
   // one row per thread leaves most of the GPU idle on small bases: the steps
-  // spread over grid columns (60 x 200 steps in turn 545 us, 16 columns 60 us)
+  // spread over grid columns (60 CTAs with 200 steps in turn 545 us, 16 columns 112 us)
   const int cols = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(K, 16), 8 * (int64_t)sms / grid));
   k_step_bounds<<<dim3(grid, cols), 256, 0, ctx->stream>>>(el::basis_dev(h->basis), h->d_diagV64, sh, K, d_om, d_dl, d_out);
   ctx->launches++;

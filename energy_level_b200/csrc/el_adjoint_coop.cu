@@ -10,14 +10,14 @@
 // pulse gradient runs on hold tens of thousands of rows, so the separate
 // launches of the stream path (about 3 K M of them) cost more than their
 // work.  A phase is a barrier and a chain of L2 reads whatever it computes
-// (2.0 us on 15,127 rows), so their number counts: the forward pass keeps
-// every term t_m of every step while all of them fit STORE_MAX bytes (318 MB
+// (2.3 us on 15,127 rows), so their number counts: the forward pass keeps
+// every term t_m of every step while all of them fit STORE_MAX bytes (363 MB
 // for 200 steps on that basis; otherwise the reverse pass forms them again
-// from the step's checkpoint, another 1827 of 7186 phases), a step's last
-// reverse phase also writes lambda and the next step's u_M, and each thread
-// adds up its gradient dots over a step, one block sum per step.  20-site
-// ring, 200 steps, complex64: 22.8 -> 10.5 ms (14.9 with the row values read
-// from memory in each phase).  Four lanes share a row (its
+// from the step's checkpoint, another 2127 phases on top of 4656), a step's
+// last reverse phase also writes lambda and the next step's u_M (400 phases
+// less), and each thread adds up its gradient dots over a step, one block sum
+// per step.  20-site ring, 200 steps, complex64: 22.8 -> 10.5 ms (14.9 with
+// the row values read from memory in each phase).  Four lanes share a row (its
 // flips split between them) as in k_adjoint_step, and keep its flip targets
 // in registers across all sweeps; every step's Chebyshev plan (a, b, M, c_m)
 // is computed on the host first and read from device arrays.  Gradient dots

@@ -171,8 +171,9 @@ __global__ void __launch_bounds__(256) k_obs_sum(int nparts, int K, const double
 // thread has every 64th row and a group of 8 sites; site sums in registers,
 // a_k of pairs in shared memory), then 36
 // blocks of 4 x 4 sites (i-block <= j-block), each shared by 7 threads with
-// their share of the rows, add their 16 pairs in FP64 registers.  Bound: FP64
-// multiply-adds (4 per pair and row).  31-site chain (dim 3,524,578,
+// their share of the rows, add their 16 pairs in FP64 registers.  Bound: instruction
+// issue, most of it the FP64 multiply-adds (4 per pair and row), at 16 warps
+// per SM (24-site chain: issue 46 %, FP64 pipe 35 %).  31-site chain (dim 3,524,578,
 // complex64), 465 pairs: 13.7 ms with an item per pair, 2.1 here; sites
 // alone 0.83 -> 0.52 ms.
 constexpr int obs_rows(bool pairs) { return pairs ? 128 : 256; }   // rows per stage
