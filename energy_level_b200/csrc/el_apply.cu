@@ -1125,9 +1125,12 @@ namespace {
 
 // Rows below which one vector goes to the row kernel: a launch is then all
 // latency, and the row kernel's chain (its gathers) is shorter than the tiled
-// kernels' (tile, barrier, gathers).  Full basis, complex128: n = 14 4.5
-// against 6.3 us, 15 6.2 against 6.5, 16 10.3 against 7.2.  Chains, float64:
-// n = 18 4.7 against 8.3, 22 8.3 against 10.3, 23 (75,025 rows) 10.3 both.
+// kernels' (tile, barrier, gathers).  Full basis, row against tiled kernel
+// alone (torch profiler): n = 15 3.1 against 4.8 us in float32, 3.4 and 5.0
+// float64, 3.8 and 5.0 complex64, 4.9 and 5.4 complex128; n = 16 4.3 and 5.1,
+// 5.3 and 5.3, 5.7 and 5.3, 8.4 and 5.8; n = 17 7.2 and 5.4, 15.0 and 6.2.
+// Chains, float64: n = 18 4.7 against 8.3 us, 22 8.3 against 10.3, 23 (75,025
+// rows) 10.3 both.
 constexpr int64_t ROW_FULL = 1 << 16, ROW_SECTOR = 75776;
 constexpr int ROW_LANES = 4;
 
